@@ -267,6 +267,10 @@ struct DevBuf {
     return e;
   }
   void release() { if (ptr) cudaFree(ptr); ptr = nullptr; cap = 0; }
+  DevBuf() = default;
+  DevBuf(const DevBuf &) = delete;
+  DevBuf &operator=(const DevBuf &) = delete;
+  ~DevBuf() { release(); }
 };
 
 }  // namespace
@@ -445,18 +449,6 @@ extern "C" int vqemps_destroy(vqemps_ctx *ctx) {
   cudaSetDevice(ctx->device);
   ctx->hams.clear();
   ctx->parts.clear();
-  ctx->sites.release(); ctx->right.release(); ctx->env0.release(); ctx->env1.release();
-  ctx->env2.release(); ctx->env3.release(); ctx->sites_t.release();
-  ctx->bonds_ws.release(); ctx->status.release(); ctx->leafval.release();
-  ctx->theta_stage.release(); ctx->energy_stage.release(); ctx->per_term_stage.release();
-  ctx->bits.release(); ctx->zsum.release(); ctx->seeds.release(); ctx->branch.release();
-  ctx->analytic_stage.release();
-  ctx->grad_sites.release(); ctx->grad_envs.release(); ctx->grad_bar0.release();
-  ctx->grad_bar1.release(); ctx->grad_sitebar.release(); ctx->grad_stage.release();
-  ctx->grad_partial.release(); ctx->grad_leafsum.release(); ctx->grad_seg.release();
-  ctx->grad_sites_t.release(); ctx->grad_senv.release(); ctx->grad_sbar0.release();
-  ctx->grad_sbar1.release(); ctx->grad_rootbar.release(); ctx->grad_partial_s.release();
-  ctx->grad_fstate.release();
   delete ctx;
   return VQEMPS_OK;
 }
