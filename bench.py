@@ -3,8 +3,8 @@
 Workload: 40 qubits, reverse_linear RY ansatz with 4 layers + final RY layer
 (200 angles), 5,000-term seeded synthetic Pauli sum (weight <= 6, 90 % Z words,
 20 % +-U(100, 1000) penalty coefficients), B = 256 parameter sets per step (SPSA
-+-0.1 probe pairs around a seeded point). One step = prepare the 256 MPS states
-(SVD gate chain) and evaluate all 5,000 terms on each: 256 energy evaluations.
++-0.1 probe pairs around a seeded point). One step = evaluate all 5,000 terms on
+each of the 256 states from their angles: 256 energy evaluations.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--batch B] [--impl ours|reference]
 
@@ -79,6 +79,54 @@ def barrier(dist, device):
         import torch
         t = torch.zeros(1, device=device)
         dist.all_reduce(t)
+
+
+class NvmlSampler:
+    """Clock and throttle reasons read through NVML every 2 ms in a thread (reads only):
+    the timed region may be shorter than nvidia-smi's sampling interval."""
+
+    REASONS = (("hw_slowdown", 0x8), ("hw_thermal_slowdown", 0x40), ("sw_thermal_slowdown", 0x20),
+               ("sw_power_cap", 0x4))
+
+    def __init__(self, index):
+        import threading
+        import pynvml
+        pynvml.nvmlInit()
+        self.nvml = pynvml
+        self.dev = pynvml.nvmlDeviceGetHandleByIndex(index)
+        self.rows = []
+        self.stopped = threading.Event()
+        self.thread = threading.Thread(target=self._run, daemon=True)
+
+    def _run(self):
+        import datetime
+        while not self.stopped.is_set():
+            self.rows.append((datetime.datetime.now(),
+                              self.nvml.nvmlDeviceGetClockInfo(self.dev, self.nvml.NVML_CLOCK_SM),
+                              self.nvml.nvmlDeviceGetCurrentClocksThrottleReasons(self.dev)))
+            self.stopped.wait(0.002)
+
+    def start(self):
+        self.thread.start()
+
+    def window(self, t0, t1):
+        self.t0, self.t1 = t0, t1
+
+    def stop(self):
+        self.stopped.set()
+        self.thread.join(timeout=10)
+        kept = [r for r in self.rows if self.t0 <= r[0] <= self.t1]
+        return dict(sm_mhz=float(np.median([r[1] for r in kept])) if kept else None,
+                    sm_max_mhz=float(self.nvml.nvmlDeviceGetMaxClockInfo(self.dev, self.nvml.NVML_CLOCK_SM)),
+                    reasons=sorted({name for r in kept for name, bit in self.REASONS if r[2] & bit}),
+                    samples=len(kept))
+
+
+def clock_sampler(index):
+    try:
+        return NvmlSampler(index)
+    except Exception:        # no NVML binding: nvidia-smi
+        return ClockSampler(index)
 
 
 class ClockSampler:
@@ -266,7 +314,7 @@ def main():
     for _ in range(args.warmup):
         step()
     torch.cuda.synchronize()
-    clocks = ClockSampler(local)
+    clocks = clock_sampler(local)
     barrier(dist, device)
     torch.cuda.synchronize()
     clocks.start()
@@ -297,6 +345,9 @@ def main():
     # multiply-add); the real-arithmetic kernel does one real multiply-add (2
     # flops) where they do a complex one
     flops_eval = stats["flops"] / 4.0 if variant == "real_pf" else stats["flops"]
+    ladder = eng.ladder_info(ham, args.batch) if variant == "ladder" else None
+    if ladder:
+        flops_eval = ladder["flops"]
     flops_step = flops_eval * args.batch
     achieved = flops_step / level_s / 1e12
     kernel = {"simt": "level_kernel (FP64 FMA pipes)", "simt_pf": "level_pf_kernel (FP64 FMA pipes, cp.async prefetch)",
@@ -306,13 +357,15 @@ def main():
               "dmma3_pf": "level_mma3_pf_kernel (FP64 DMMA tensor cores, Gauss 3-product complex multiply, "
                           "cp.async parent prefetch)",
               "real_pf": "level_real_pf_kernel (FP64 DMMA tensor cores, real arithmetic with Y-count phases for "
-                         "real-amplitude states, 1-D bulk-copy staging on mbarriers)"}.get(variant, str(variant))
+                         "real-amplitude states, 1-D bulk-copy staging on mbarriers)",
+              "ladder": "ladder_path_kernel (FP64 FMA pipes, environments as Pauli components in registers) and "
+                        "ladder_close_kernel"}.get(variant, str(variant))
     traffic = profiled_traffic(variant)
-    roofline = dict(bound="tensor" if variant and variant != "simt" and variant != "simt_pf" else "fp64",
+    roofline = dict(bound="tensor" if variant and variant not in ("simt", "simt_pf", "ladder") else "fp64",
                     achieved=achieved,
                     peak=fp64_peak, unit="TFLOP/s", frac=achieved / fp64_peak,
                     traffic=traffic * args.batch if traffic else None,
-                    kernel=kernel + ", all trie levels of one step",
+                    kernel=kernel + (", all paths and closures of one step" if ladder else ", all trie levels of one step"),
                     peak_source="cuBLAS FP64 DGEMM 8192^3 (DMMA tensor cores) measured in this run, burst",
                     survey_unit_tflops=stats["flops_survey"] * args.batch / level_s / 1e12)
 
@@ -353,10 +406,10 @@ def main():
                     ms_per_step=ms_per_step, higher_is_better=True, scaling="weak", vs_baseline=None,
                     dtype="f64", data="synthetic",
                     config=dict(WORKLOAD, global_batch=args.batch * world, parallelism=f"replicas x{world}",
-                                l2="working set per step > L2 (level environments ~6 GB): no flush needed",
+                                l2="working set per step > L2 (environments > 1 GB): no flush needed",
                                 plain_evals_per_s=plain_rate, batched_over_plain=value / world / plain_rate,
                                 flops_per_eval=flops_eval, survey_flops_per_eval=stats["flops_survey"],
-                                trie_node_sites=stats["node_sites"],
+                                trie_node_sites=ladder["steps"] if ladder else stats["node_sites"],
                                 phases_ms=phases["ms"], golden_gate=gate),
                     roofline=roofline, cpu_baseline=cpu, e2e=e2e,
                     gpu_launches=phases["launches_per_step"] * args.steps,

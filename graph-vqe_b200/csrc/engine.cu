@@ -24,8 +24,11 @@
 #include "sample.cuh"
 #include "gradient.cuh"
 #include "gradient_mma.cuh"
+#include "ladder.cuh"
 
 using namespace vqemps;
+
+#include "ladder_plan.inc"
 
 namespace {
 
@@ -53,6 +56,8 @@ struct Hamiltonian {
   std::vector<uint8_t> codes;            // T x n site-order Pauli codes
   std::vector<double> coeffs;            // T
   int nzwords = 0;                       // non-identity I/Z words (independent streams)
+  bool split_allowed = true;             // loaded with split evaluation allowed
+  std::unique_ptr<LadderPlan> ladder;    // built on the first call of a ladder circuit
   // device copies
   DevGroup *d_groups = nullptr;
   DevNode *d_nodes = nullptr;
@@ -279,7 +284,8 @@ struct DevBuf {
 enum : int {
   LV_SIMT4 = 0, LV_MMA4 = 1, LV_MMA8 = 2, LV_PF4 = 3, LV_MMAPF4 = 4, LV_MMA3PF4 = 5,
   LV_REALPF4 = 6,   // real arithmetic: circuits of real gates only
-  LV_COUNT = 7
+  LV_LADDER = 7,    // Pauli components, ladder circuits only: a rule, not a candidate (ladder.cuh)
+  LV_COUNT = 8
 };
 
 struct vqemps_ctx {
@@ -307,6 +313,9 @@ struct vqemps_ctx {
   cplx *d_mats = nullptr;
   SiteEvent *d_events = nullptr;
   int32_t *d_ev_off = nullptr, *d_ev_dims = nullptr, *d_slot_off = nullptr, *d_slot_list = nullptr;
+  LadderCircuit ladder;                 // the circuit as a ladder (ladder_plan.inc)
+  LadGate *d_lad_gates = nullptr;
+  int32_t *d_lad_off = nullptr;
   // hamiltonians
   std::map<int, std::unique_ptr<Hamiltonian>> hams;
   std::map<int, std::unique_ptr<PartSet>> parts;
@@ -338,6 +347,11 @@ struct vqemps_ctx {
   // second stream) and the left sweep's F at the cut
   DevBuf<cplx> grad_sites_t, grad_senv, grad_sbar0, grad_sbar1, grad_rootbar, grad_partial_s, grad_fstate;
   DevBuf<double> grad_stage;
+  DevBuf<double> lad_coef, lad_poison, lad_envp, lad_envs, lad_theta;
+  int ladder_list = -1;                 // task list of the ladder kernels, -1: by batch size
+  int ladder_launches = 0;              // kernels the last run_ladder launched
+  int ladder_B = 0;                     // > 0: the last energies came from the ladder kernels, which prepare no
+                                        // site tensors; angles of that many states are in lad_theta
   int last_B = 0;
   int forced_variant = -1;              // level kernel variant, -1: autotune
   // Autotuner decisions shared by plans of one size class: (batch-size bucket,
@@ -357,6 +371,7 @@ struct vqemps_ctx {
   ~vqemps_ctx() {
     cudaFree(d_gates); cudaFree(d_mats); cudaFree(d_events); cudaFree(d_ev_off);
     cudaFree(d_ev_dims); cudaFree(d_slot_off); cudaFree(d_slot_list);
+    cudaFree(d_lad_gates); cudaFree(d_lad_off);
     cudaFree(d_sched); cudaFree(d_gate_q); cudaFree(d_qlist); cudaFree(d_tail_off); cudaFree(d_qsched);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
@@ -433,10 +448,13 @@ extern "C" int vqemps_create(int device, int max_bond, double abs_cut, double re
                        (int)sizeof(GradBwdRealSmem));
   if (const char *v = std::getenv("VQEMPS_GRAD_VARIANT"))
     ctx->grad_mma = std::strcmp(v, "simt") == 0 ? 0 : std::strcmp(v, "dmma") == 0 ? 1 : 2;
+  if (const char *v = std::getenv("VQEMPS_LADDER_LIST"))
+    if (v[0] >= '0' && v[0] < '0' + LAD_LISTS && v[1] == 0) ctx->ladder_list = v[0] - '0';
   // VQEMPS_LEVEL_VARIANT pins the trie-level kernel (a name or an index); the
   // autotuner's timings are meaningless under a serialising profiler.
   if (const char *v = std::getenv("VQEMPS_LEVEL_VARIANT")) {
-    static const char *names[LV_COUNT] = {"simt", "dmma4", "dmma8", "simt_pf", "dmma_pf", "dmma3_pf", "real_pf"};
+    static const char *names[LV_COUNT] = {"simt", "dmma4", "dmma8", "simt_pf", "dmma_pf", "dmma3_pf", "real_pf",
+                                           "ladder"};
     for (int i = 0; i < LV_COUNT; ++i)
       if (std::strcmp(v, names[i]) == 0 || (v[0] == '0' + i && v[1] == 0)) ctx->forced_variant = i;
   }
@@ -520,6 +538,7 @@ extern "C" int vqemps_set_circuit(vqemps_ctx *ctx, int n, const vqemps_op *ops, 
   std::vector<int> bonds(n + 1, 1);
   int P = 0;
   bool doubling_ok = true;
+  bool named = true;       // no user-supplied matrices (every one-site gate is unitary to rounding)
   bool real = true;        // RY, H, X, Z, CX, SWAP and real U1 / U2 matrices keep amplitudes real
   const int maxb = ctx->max_bond;
   auto add_two = [&](int s, int mat) {
@@ -556,6 +575,7 @@ extern "C" int vqemps_set_circuit(vqemps_ctx *ctx, int n, const vqemps_op *ops, 
           if (m[i].y != 0.0) real = false;
         push_matrix(mats, m, 4, &g.mat);
         go.mat = g.mat;
+        named = false;
       } else {
         g.mat = fixed_off[op.kind - VQEMPS_H];
         go.mat = g.mat;
@@ -643,6 +663,18 @@ extern "C" int vqemps_set_circuit(vqemps_ctx *ctx, int n, const vqemps_op *ops, 
     CUDA_TRY(ctx, upi(ctx->d_qsched, qs.sched));
     ctx->qsteps = qs.nsteps;
   }
+  ctx->ladder = doubling_ok && named ? compile_ladder(n, gops, real) : LadderCircuit{};
+  ctx->ladder_B = 0;
+  if (ctx->ladder.ok) {
+    const LadderCircuit &lc = ctx->ladder;
+    cudaFree(ctx->d_lad_gates); ctx->d_lad_gates = nullptr;
+    cudaFree(ctx->d_lad_off); ctx->d_lad_off = nullptr;
+    CUDA_TRY(ctx, cudaMalloc(&ctx->d_lad_gates, std::max<size_t>(lc.gates.size(), 1) * sizeof(LadGate)));
+    CUDA_TRY(ctx, cudaMalloc(&ctx->d_lad_off, lc.off.size() * sizeof(int32_t)));
+    if (!lc.gates.empty())
+      CUDA_TRY(ctx, cudaMemcpy(ctx->d_lad_gates, lc.gates.data(), lc.gates.size() * sizeof(LadGate), cudaMemcpyHostToDevice));
+    CUDA_TRY(ctx, cudaMemcpy(ctx->d_lad_off, lc.off.data(), lc.off.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+  }
   ctx->gates = std::move(gates);
   ctx->mats = std::move(mats);
   ctx->grad_ops = std::move(gops);
@@ -699,6 +731,7 @@ extern "C" int vqemps_set_hamiltonian(vqemps_ctx *ctx, const char *words, const 
   auto h = std::make_unique<Hamiltonian>();
   h->n = n;
   h->T = T;
+  h->split_allowed = ctx->split_mode != 0;
   // site-order codes (buildPauliTermData reverses words for the msb map)
   std::vector<uint8_t> code((size_t)T * n);
   std::vector<int> last(T, -1);
@@ -1078,6 +1111,7 @@ static bool use_quad_chain(vqemps_ctx *ctx, int B) {
 }
 
 static int launch_evolve(vqemps_ctx *ctx, const double *theta_dev, int B, cudaStream_t st) {
+  ctx->ladder_B = 0;
   EvolveParams ep{};
   ep.gates = ctx->d_gates;
   ep.ngates = (int)ctx->gates.size();
@@ -1363,6 +1397,8 @@ static int run_levels_mcut(vqemps_ctx *ctx, Hamiltonian &h, int B, cudaStream_t 
 }
 
 static int run_levels(vqemps_ctx *ctx, Hamiltonian &h, int B, cudaStream_t st, int variant) {
+  if (variant == LV_LADDER)
+    return fail(ctx, VQEMPS_INVALID, "the ladder kernels need a ladder circuit (vqemps_set_level_variant)");
   if (variant == LV_REALPF4 && !ctx->real_circuit)
     return fail(ctx, VQEMPS_INVALID, "the real-arithmetic level kernels need a circuit of real gates");
   if (h.mcut) return run_levels_mcut(ctx, h, B, st, variant);
@@ -1514,7 +1550,7 @@ static int pick_variant(vqemps_ctx *ctx, Hamiltonian &h, int B, cudaStream_t st,
   CUDA_TRY(ctx, cudaEventCreate(&ev.e1));
   int best = LV_SIMT4;
   float best_ms = 1e30f;
-  for (int v = 0; v < LV_COUNT; ++v) {
+  for (int v = 0; v < LV_LADDER; ++v) {
     if (v == LV_REALPF4 && !ctx->real_circuit) continue;   // complex amplitudes
     int rc = run_levels(ctx, h, B, st, v);      // warm
     if (rc) return rc;
@@ -1595,11 +1631,14 @@ static Hamiltonian *find_ham(vqemps_ctx *ctx, int handle) {
   return it == ctx->hams.end() ? nullptr : it->second.get();
 }
 
+#include "engine_ladder.inc"
+
 extern "C" int vqemps_level_variant(vqemps_ctx *ctx, int handle, int B, int *variant) {
   if (!ctx || !variant) return VQEMPS_INVALID;
   Hamiltonian *h = find_ham(ctx, handle);
   if (!h) return VQEMPS_INVALID;
   if (ctx->forced_variant >= 0) { *variant = ctx->forced_variant; return VQEMPS_OK; }
+  if (use_ladder(ctx, h)) { *variant = LV_LADDER; return VQEMPS_OK; }
   auto it = h->tuned.find(batch_bucket(B));
   *variant = it == h->tuned.end() ? -1 : it->second;
   return VQEMPS_OK;
@@ -1615,6 +1654,12 @@ extern "C" int vqemps_energy_batch(vqemps_ctx *ctx, int handle, const double *th
     return fail(ctx, VQEMPS_INVALID, "bad batch arguments");
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = as_stream(stream);
+  if (use_ladder(ctx, h)) {
+    const int rc = run_ladder(ctx, h, theta_dev, B, energies_dev, per_term_dev, st, nullptr);
+    if (rc) return rc;
+    ctx->ladder_B = ctx->last_B = B;
+    return VQEMPS_OK;
+  }
   int rc = select_plan(ctx, h, B);
   if (rc) return rc;
   rc = ensure_state_ws(ctx, B);
@@ -1639,12 +1684,29 @@ extern "C" int vqemps_profile_energy(vqemps_ctx *ctx, int handle, const double *
   if (!h || B < 1) return fail(ctx, VQEMPS_INVALID, "bad profile arguments");
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = as_stream(stream);
+  CUDA_TRY(ctx, ctx->energy_stage.ensure((size_t)B));
+  cudaEvent_t ev[5];
+  if (use_ladder(ctx, h)) {
+    // preparation = the rotations, no right environments, levels = paths and closures
+    for (auto &e : ev) CUDA_TRY(ctx, cudaEventCreate(&e));
+    const int rc = run_ladder(ctx, h, theta_dev, B, ctx->energy_stage.ptr, nullptr, st, ev);
+    if (rc) return rc;
+    CUDA_TRY(ctx, cudaEventSynchronize(ev[3]));
+    float t[3];
+    for (int i = 0; i < 3; ++i) CUDA_TRY(ctx, cudaEventElapsedTime(&t[i], ev[i], ev[i + 1]));
+    ms[0] = t[0];
+    ms[1] = 0.0;
+    ms[2] = t[1];
+    ms[3] = t[2];
+    *launches = ctx->ladder_launches;
+    for (auto &e : ev) cudaEventDestroy(e);
+    ctx->ladder_B = ctx->last_B = B;
+    return VQEMPS_OK;
+  }
   int rc = select_plan(ctx, h, B);
   if (rc) return rc;
   rc = ensure_state_ws(ctx, B);
   if (rc) return rc;
-  CUDA_TRY(ctx, ctx->energy_stage.ensure((size_t)B));
-  cudaEvent_t ev[5];
   for (auto &e : ev) CUDA_TRY(ctx, cudaEventCreate(&e));
   CUDA_TRY(ctx, cudaEventRecord(ev[0], st));
   rc = launch_evolve(ctx, theta_dev, B, st);
@@ -1726,6 +1788,13 @@ extern "C" int vqemps_copy_sites(vqemps_ctx *ctx, int b, double *sites_host, voi
   if (!ctx || !sites_host || b < 0 || b >= ctx->last_B) return VQEMPS_INVALID;
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = as_stream(stream);
+  if (ctx->ladder_B > 0) {              // the last energies prepared no site tensors: run the gate chain now
+    if (b >= ctx->ladder_B) return VQEMPS_INVALID;
+    const int rc0 = ensure_state_ws(ctx, ctx->ladder_B);
+    if (rc0) return rc0;
+    const int rc = launch_evolve(ctx, ctx->lad_theta.ptr, ctx->ladder_B, st);
+    if (rc) return rc;
+  }
   CUDA_TRY(ctx, cudaMemcpyAsync(sites_host, ctx->sites.ptr + (size_t)b * ctx->n * SITE_ELEMS,
                                 sizeof(cplx) * ctx->n * SITE_ELEMS, cudaMemcpyDeviceToHost, st));
   CUDA_TRY(ctx, cudaStreamSynchronize(st));

@@ -26,7 +26,8 @@ SYMBOLS = (
     "vqemps_num_params", "vqemps_bond_dims", "vqemps_set_hamiltonian",
     "vqemps_free_hamiltonian", "vqemps_energy_batch", "vqemps_energy_batch_host",
     "vqemps_batch_status", "vqemps_energy_grad_batch", "vqemps_sample",
-    "vqemps_sampled_energy", "vqemps_copy_sites", "vqemps_plan_stats", "vqemps_profile_energy",
+    "vqemps_sampled_energy", "vqemps_copy_sites", "vqemps_plan_stats", "vqemps_ladder_info",
+    "vqemps_profile_energy",
     "vqemps_energy_noalloc", "vqemps_set_level_variant", "vqemps_level_variant",
     "vqemps_set_grad_checkpoint", "vqemps_set_grad_variant", "vqemps_set_split_mode", "vqemps_set_evolve_mode",
     "vqemps_set_partitions", "vqemps_free_partitions",
@@ -90,6 +91,7 @@ def load():
         "vqemps_sampled_energy": (I, [P, I, V, I, I, u64, I, I, V, V, V]),
         "vqemps_copy_sites": (I, [P, I, ctypes.POINTER(D), V]),
         "vqemps_plan_stats": (I, [P, I, ctypes.POINTER(D)]),
+        "vqemps_ladder_info": (I, [P, I, I, ctypes.POINTER(D)]),
         "vqemps_profile_energy": (I, [P, I, V, I, ctypes.POINTER(D), ctypes.POINTER(I), V]),
         "vqemps_energy_noalloc": (I, [P, I, V, V, V, V, V]),
         "vqemps_set_level_variant": (I, [P, I]),

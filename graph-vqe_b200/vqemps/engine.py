@@ -201,8 +201,9 @@ class Engine:
     def free_hamiltonian(self, ham: Hamiltonian):
         check(self.ctx, self.lib.vqemps_free_hamiltonian(self.ctx, ham.handle), "free_hamiltonian")
 
-    # "real_pf": real arithmetic, for circuits of real gates only
-    LEVEL_VARIANTS = ("simt", "dmma4", "dmma8", "simt_pf", "dmma_pf", "dmma3_pf", "real_pf")
+    # "real_pf": real arithmetic, for circuits of real gates only; "ladder": Pauli
+    # components, for the circuits of include/vqemps.h (the default there)
+    LEVEL_VARIANTS = ("simt", "dmma4", "dmma8", "simt_pf", "dmma_pf", "dmma3_pf", "real_pf", "ladder")
 
     def set_level_variant(self, variant):
         """Force a trie-level kernel (one of LEVEL_VARIANTS) or None to autotune."""
@@ -221,12 +222,19 @@ class Engine:
                 "prefix_flops", "prefix_node_sites", "pairs")
         return dict(zip(keys, list(out)))
 
+    def ladder_info(self, ham: Hamiltonian, B: int) -> dict:
+        """Per-state work of an energy call of B states with the ladder kernels."""
+        out = (ctypes.c_double * 4)()
+        check(self.ctx, self.lib.vqemps_ladder_info(self.ctx, ham.handle, B, out), "ladder_info")
+        return dict(zip(("steps", "closures", "flops", "slots"), list(out)))
+
     def set_evolve_mode(self, mode: str):
         """Gate chain: 'quad' (four-CTA clusters, circuits of real gates; others run
         'pair'), 'pair' (two-CTA clusters on a schedule), 'chain' (one CTA, program
         order) or 'auto' (default: quad for a circuit of real gates while all its
         clusters fit the GPU at once, else pair while the batch has at most two
-        states per SM, else chain). All give the same states bit for bit."""
+        states per SM, else chain). All give the same states bit for bit. With
+        'auto', energies of ladder circuits run no chain at all (include/vqemps.h)."""
         check(self.ctx, self.lib.vqemps_set_evolve_mode(
             self.ctx, {"chain": 0, "pair": 1, "quad": 2, "auto": -1}[mode]), "set_evolve_mode")
 

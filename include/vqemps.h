@@ -184,14 +184,24 @@ int vqemps_sampled_energy(vqemps_ctx *ctx, int handle, const double *theta_dev, 
  * vqemps_set_level_variant forces one (-1 restores tuning);
  * vqemps_level_variant reports the one in use (-1: not tuned yet). The
  * environment variable VQEMPS_LEVEL_VARIANT (simt, dmma4, dmma8, simt_pf,
- * dmma_pf, dmma3_pf or 0-5), read by vqemps_create, forces one for every context. */
+ * dmma_pf, dmma3_pf or 0-5), read by vqemps_create, forces one for every context.
+ * Two more serve special circuits: 6 real_pf (circuits of real gates, a tuning
+ * candidate) and 7 ladder. Ladder circuits -- layers of named one-site gates, each
+ * followed by one CX on every bond in chain order, all in one direction, at most
+ * four layers (the linear and reverse_linear ansatz) -- have an exact matrix
+ * product state that needs no SVD. With no variant or gate chain forced, zero
+ * cutoffs, 2^layers <= max_bond and split evaluation not switched off, their
+ * energies are evaluated from it without preparing site tensors (variant 7;
+ * equal to the others to rounding, 1e-12 per term). VQEMPS_LADDER_LIST (0, 1
+ * or 2), read by vqemps_create, forces one of its task lists (same bits). */
 int vqemps_set_level_variant(vqemps_ctx *ctx, int variant);
 int vqemps_level_variant(vqemps_ctx *ctx, int handle, int B, int *variant);
 
 /* Benchmark support (no reference counterpart): phase times of one batched
  * energy call -- ms[0] state preparation, ms[1] right environments, ms[2] trie
  * levels, ms[3] energy reduction -- and the number of kernels one call launches.
- * Synchronises the stream. */
+ * With the ladder kernels ms[0] is the rotations and ms[1] zero. Synchronises the
+ * stream. */
 int vqemps_profile_energy(vqemps_ctx *ctx, int handle, const double *theta_dev, int B, double *ms,
                           int *launches, void *stream);
 
@@ -204,6 +214,11 @@ int vqemps_profile_energy(vqemps_ctx *ctx, int handle, const double *theta_dev, 
  * fewer node-sites), [7] / [8] flops / node-sites of the prefix trie alone,
  * [9] prefix/suffix pair closures. */
 int vqemps_plan_stats(const vqemps_ctx *ctx, int handle, double *stats);
+
+/* Work of an energy call of B states with the ladder kernels, per state (info[4]):
+ * steps walked, closures, FP64 operations of the steps, environment slots.
+ * VQEMPS_INVALID when such a call would not run them. */
+int vqemps_ladder_info(vqemps_ctx *ctx, int handle, int B, double *info);
 
 /* Split evaluation (no reference counterpart; the reference walks prefix tries
  * only, sharded_mps.cuh:614-687): a Pauli sum loaded afterwards is evaluated as
@@ -221,13 +236,15 @@ int vqemps_set_split_mode(vqemps_ctx *ctx, int mode);
  * CTA per state in program order; -1 (default) uses 2 for a circuit of real gates
  * while all clusters of four fit the GPU at once and the four-gate schedule is
  * shorter, else 1 while the batch has at most twice as many states as the GPU has
- * SMs, else 0. All give the same states bit for bit. */
+ * SMs, else 0. All give the same states bit for bit.
+ * Energies of ladder circuits (vqemps_set_level_variant) run no chain at -1. */
 int vqemps_set_evolve_mode(vqemps_ctx *ctx, int mode);
 
 /* Copy the site tensors of state b of the last batched call to the host:
  * n * 16 * 2 * 16 complex (re, im) pairs, site s at offset s * 1024 doubles,
  * element (l, p, r) at ((l * 2 + p) * 16 + r), zero padded beyond the bond dims.
- * Used to check the prepared state against the oracle (synchronises). */
+ * Used to check the prepared state against the oracle (synchronises). After
+ * energies of a ladder circuit the gate chain runs here, on the call's angles. */
 int vqemps_copy_sites(vqemps_ctx *ctx, int b, double *sites_host, void *stream);
 
 /* Partition sets: K independent circuits of uneven width, parameter count and
