@@ -25,10 +25,12 @@
 #include "gradient.cuh"
 #include "gradient_mma.cuh"
 #include "ladder.cuh"
+#include "ladder_grad.cuh"
 
 using namespace vqemps;
 
 #include "ladder_plan.inc"
+#include "ladder_grad_plan.inc"
 
 namespace {
 
@@ -348,6 +350,7 @@ struct vqemps_ctx {
   DevBuf<cplx> grad_sites_t, grad_senv, grad_sbar0, grad_sbar1, grad_rootbar, grad_partial_s, grad_fstate;
   DevBuf<double> grad_stage;
   DevBuf<double> lad_coef, lad_poison, lad_envp, lad_envs, lad_theta;
+  DevBuf<double> lad_cotp, lad_cots, lad_part, lad_sums;   // ladder gradients
   int ladder_list = -1;                 // task list of the ladder kernels, -1: by batch size
   int ladder_launches = 0;              // kernels the last run_ladder launched
   int ladder_B = 0;                     // > 0: the last energies came from the ladder kernels, which prepare no
@@ -359,6 +362,7 @@ struct vqemps_ctx {
   std::map<int, int> tuned_by_shape;
   int grad_checkpoint = 8;              // gradient: keep every 8th level's environments
   int grad_mma = 2;                     // gradient levels: 0 SIMT, 1 FP64 DMMA, 2 DMMA with Gauss forward
+  bool grad_default = true;             // no gradient variant asked for: ladder circuits take the ladder kernels
   int split_mode = -1;                  // split evaluation: -1 when it saves work, 0 never, 1 always
   int evolve_pair = -1;                 // gate chain: 2 four-CTA clusters (real circuits), 1 two-CTA
                                         // clusters, 0 one CTA, -1 by batch size
@@ -435,6 +439,8 @@ extern "C" int vqemps_create(int device, int max_bond, double abs_cut, double re
                        (int)sizeof(LevelMmaPfSmem));
   cudaFuncSetAttribute(level_mma3_pf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(LevelMmaPfSmem));
+  cudaFuncSetAttribute(ladder_back_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lad_back_smem<true>());
+  cudaFuncSetAttribute(ladder_back_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lad_back_smem<false>());
   grad_set_attributes();
   cudaFuncSetAttribute(grad_fwd_level_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(GradFwdMmaSmem));
@@ -446,8 +452,10 @@ extern "C" int vqemps_create(int device, int max_bond, double abs_cut, double re
                        (int)sizeof(GradFwdRealSmem));
   cudaFuncSetAttribute(grad_bwd_level_real_a_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(GradBwdRealSmem));
-  if (const char *v = std::getenv("VQEMPS_GRAD_VARIANT"))
+  if (const char *v = std::getenv("VQEMPS_GRAD_VARIANT")) {
     ctx->grad_mma = std::strcmp(v, "simt") == 0 ? 0 : std::strcmp(v, "dmma") == 0 ? 1 : 2;
+    ctx->grad_default = false;
+  }
   if (const char *v = std::getenv("VQEMPS_LADDER_LIST"))
     if (v[0] >= '0' && v[0] < '0' + LAD_LISTS && v[1] == 0) ctx->ladder_list = v[0] - '0';
   // VQEMPS_LEVEL_VARIANT pins the trie-level kernel (a name or an index); the
@@ -1802,6 +1810,7 @@ extern "C" int vqemps_copy_sites(vqemps_ctx *ctx, int b, double *sites_host, voi
 }
 
 #include "engine_sample.inc"
+#include "engine_ladder_grad.inc"
 #include "engine_grad.inc"
 #include "engine_parts.inc"
 #include "noalloc.cu"

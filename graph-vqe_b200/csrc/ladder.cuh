@@ -45,7 +45,8 @@ constexpr int LAD_COEFS = 40;        // n | k = 2, 3, 4: O row-major | W row-maj
 constexpr int LAD_MAX_LAYERS = 4;
 
 struct LadGate {   // a one-site gate of a layer: fixed matrix or rotation
-  int32_t mat, rot, param, pad;
+  int32_t mat, rot, param;
+  int32_t slot;            // index of its angle derivative, -1 without a parameter
   double angle;
 };
 

@@ -288,7 +288,8 @@ class Engine:
         check(self.ctx, self.lib.vqemps_set_grad_checkpoint(self.ctx, int(every)), "set_grad_checkpoint")
 
     def set_grad_variant(self, variant: str):
-        """Gradient level kernels: 'dmma3' (FP64 tensor cores, Gauss forward; default), 'dmma' or 'simt'."""
+        """Gradient level kernels: 'dmma3' (FP64 tensor cores, Gauss forward), 'dmma' or 'simt'. The default is
+        the ladder kernels for ladder circuits (include/vqemps.h) and 'dmma3' for the others."""
         check(self.ctx, self.lib.vqemps_set_grad_variant(self.ctx, {"simt": 0, "dmma": 1, "dmma3": 2}[variant]),
               "set_grad_variant")
 

@@ -1,0 +1,123 @@
+"""GPU: ladder gradient kernels against the oracle's adjoint gradient, the level kernels and
+themselves. Tolerance: a derivative is a sum over words of c times a value bounded by 1
+(rotations by half angles), computed to 1e-12 like the values themselves."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import mps_oracle as O
+from oracle import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def vq(cuda_device):
+    import vqemps
+    return vqemps
+
+
+def _grad(vq, spec, words, coeffs, x, order="msb", variant=None):
+    eng = vq.Engine(0, 16)
+    if variant:
+        eng.set_grad_variant(variant)
+    eng.set_spec(spec, site_order=order)
+    e, g = eng.energy_grad(eng.set_hamiltonian(words, coeffs), np.atleast_2d(x))
+    out = e.cpu().numpy(), g.cpu().numpy()
+    eng.close()
+    return out
+
+
+@pytest.mark.parametrize("gates", [("ry",), ("ry", "rz"), ("rx", "rz")])
+@pytest.mark.parametrize("pattern", ["linear", "reverse_linear"])
+@pytest.mark.parametrize("order", ["msb", "qubit"])
+def test_ladder_gradient_matches_oracle(vq, gates, pattern, order):
+    rng = np.random.default_rng(17)
+    for n, reps, initial in ((2, 4, None), (3, 1, "+"), (5, 2, "1"), (6, 3, "-"), (9, 4, None)):
+        spec = O.hardware_efficient_spec(n, reps, gates, pattern)
+        spec["initial"] = initial
+        words, coeffs = W.random_hamiltonian(rng, n, 50, min(n, 4), z_fraction=0.4)
+        words += ["I" * n, words[0], "X" + "I" * (n - 1), "I" * (n - 1) + "Z"]
+        coeffs = np.append(coeffs, rng.normal(size=4))
+        x = rng.uniform(-np.pi, np.pi, (2, spec["count"]))
+        e, g = _grad(vq, spec, words, coeffs, x, order)
+        tol = 1e-12 * np.abs(coeffs).sum()
+        for b in range(2):
+            ref, gref = O.reverse_value_gradient(spec, words, coeffs, x[b])
+            assert abs(e[b] - ref) <= tol
+            np.testing.assert_allclose(g[b], gref, rtol=0, atol=tol)
+
+
+def test_constant_gates_scales_and_shared_parameters(vq):
+    """Fixed gates in a layer, rotations with a scale or a constant angle, a parameter used twice."""
+    rng = np.random.default_rng(23)
+    n, ops = 4, []
+    chain = [("cx", q, q + 1) for q in range(n - 1)]
+    for layer in range(2):
+        for q in range(n):
+            ops += [("h", q), ("ry", q, (layer * n + q) % 6, 0.7), ("z", q), ("rx", q, 6 + q), ("ry", q, None, 0.3), ("s", q)]
+        ops += chain
+    ops += [("rz", q, 2, -1.3) for q in range(n)]
+    words, coeffs = W.random_hamiltonian(rng, n, 30, 4, z_fraction=0.3)
+    eng = vq.Engine(0, 16)
+    eng.set_circuit(n, ops)
+    ham = eng.set_hamiltonian(words, coeffs)
+    assert eng.level_variant(ham, 1) == "ladder"
+    x = rng.uniform(-np.pi, np.pi, (3, eng.P))
+    e, g = (v.cpu().numpy() for v in eng.energy_grad(ham, x))
+    eng.set_grad_variant("dmma")
+    e0, g0 = (v.cpu().numpy() for v in eng.energy_grad(ham, x))
+    tol = 1e-11 * np.abs(coeffs).sum()
+    np.testing.assert_allclose(e, e0, rtol=0, atol=tol)
+    np.testing.assert_allclose(g, g0, rtol=0, atol=tol)
+    eng.close()
+
+
+@pytest.mark.parametrize("gates", [("ry",), ("ry", "rz")])
+def test_ladder_gradient_does_not_depend_on_batch_and_agrees_over_lists(vq, monkeypatch, gates):
+    """Within a task list the bits do not depend on the batch; lists sum a site's steps in other orders."""
+    rng = np.random.default_rng(29)
+    n = 12
+    spec = O.hardware_efficient_spec(n, 4, gates, "linear")
+    words, coeffs = W.random_hamiltonian(rng, n, 300, 5)
+    x = rng.uniform(-np.pi, np.pi, (35, spec["count"]))
+    e0, g0 = _grad(vq, spec, words, coeffs, x[:8], variant="dmma")
+    tol = 1e-11 * np.abs(coeffs).sum()
+    for name in ("0", "1", "2"):
+        monkeypatch.setenv("VQEMPS_LADDER_LIST", name)
+        e, g = _grad(vq, spec, words, coeffs, x)
+        np.testing.assert_allclose(e[:8], e0, rtol=0, atol=tol)
+        np.testing.assert_allclose(g[:8], g0, rtol=0, atol=tol)
+        for B in (1, 5, 9):
+            eb, gb = _grad(vq, spec, words, coeffs, x[:B])
+            assert np.array_equal(eb, e[:B]) and np.array_equal(gb, g[:B])
+
+
+def test_ladder_gradient_passes_split_large_batches(vq):
+    """More states than one pass holds (16 GB): 64 qubits, 20,000 words."""
+    from vqemps import workloads as VW
+    spec, words, coeffs, x = VW.gradient_64q(seed=3, batch=4)
+    eng = vq.Engine(0, 16)
+    eng.set_spec(spec)
+    ham = eng.set_hamiltonian(words, coeffs)
+    B = 150
+    e, g = eng.energy_grad(ham, torch.tensor(np.tile(x, (B // 4 + 1, 1))[:B], device=eng.device))
+    e, g = e.cpu().numpy(), g.cpu().numpy()
+    assert np.array_equal(e[:4], e[144:148]) and np.array_equal(g[:4], g[144:148])
+    eng.set_grad_variant("dmma3")
+    e0, g0 = (v.cpu().numpy() for v in eng.energy_grad(ham, x[:2]))
+    np.testing.assert_allclose(e[:2], e0, rtol=1e-10)
+    np.testing.assert_allclose(g[:2], g0, rtol=0, atol=1e-10 * np.abs(g0).max())
+    eng.close()
+
+
+def test_gradient_at_angles_that_are_not_finite(vq):
+    spec = O.hardware_efficient_spec(5, 2, ("ry",), "linear")
+    words, coeffs = ["ZZIII", "IIXXI"], np.array([1.0, 0.25])
+    x = np.random.default_rng(1).uniform(-1, 1, (3, spec["count"]))
+    good = _grad(vq, spec, words, coeffs, x)
+    x[1, 2] = np.nan
+    e, g = _grad(vq, spec, words, coeffs, x)
+    assert np.isnan(e[1]) and np.isnan(g[1]).all()
+    for b in (0, 2):
+        assert e[b] == good[0][b] and np.array_equal(g[b], good[1][b])
