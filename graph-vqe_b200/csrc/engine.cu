@@ -233,6 +233,10 @@ struct PartSet {
   int nlevels = 0;
   double flops = 0.0;                                        // one evaluation of every partition
   std::vector<int> bonds;                                    // K x (n_max + 1) allocation bounds
+  bool doubling_ok = true;              // every partition has a bond-doubling state
+  int doubled_bond = 1;
+  SiteEvent *d_events = nullptr;        // its events, K x (n_max + 1) offsets
+  int32_t *d_ev_off = nullptr;
   DevGate *d_gates = nullptr;
   cplx *d_mats = nullptr;
   DevGroup *d_groups = nullptr;
@@ -253,6 +257,7 @@ struct PartSet {
   int32_t *d_st_part = nullptr;
   int32_t *d_work = nullptr;
   ~PartSet() {
+    cudaFree(d_events); cudaFree(d_ev_off);
     cudaFree(d_gates); cudaFree(d_mats); cudaFree(d_groups); cudaFree(d_nodes); cudaFree(d_part);
     cudaFree(d_leaf_coef); cudaFree(d_term_leaf); cudaFree(d_zmask); cudaFree(d_coeffs);
     cudaFree(d_sumidx); cudaFree(d_st_part); cudaFree(d_work);
@@ -302,6 +307,7 @@ struct vqemps_ctx {
   // amplitudes and the real-arithmetic level kernels may run
   bool real_circuit = false;
   bool doubling_ok = false;             // only adjacent CX two-qubit gates (gradient path)
+  int doubled_bond = 1;                 // largest bond of the bond-doubling state
   std::vector<DevGate> gates;
   std::vector<cplx> mats;
   std::vector<int> bonds;               // zero-cutoff allocation bound, n + 1
@@ -353,8 +359,8 @@ struct vqemps_ctx {
   DevBuf<double> lad_cotp, lad_cots, lad_part, lad_sums;   // ladder gradients
   int ladder_list = -1;                 // task list of the ladder kernels, -1: by batch size
   int ladder_launches = 0;              // kernels the last run_ladder launched
-  int ladder_B = 0;                     // > 0: the last energies came from the ladder kernels, which prepare no
-                                        // site tensors; angles of that many states are in lad_theta
+  int ladder_B = 0;                     // > 0: the last call ran no gate chain (ladder kernels, bond-doubling
+                                        // states); angles of that many states are in lad_theta
   int last_B = 0;
   int forced_variant = -1;              // level kernel variant, -1: autotune
   // Autotuner decisions shared by plans of one size class: (batch-size bucket,
@@ -1118,7 +1124,8 @@ static bool use_quad_chain(vqemps_ctx *ctx, int B) {
   return B <= ctx->quad_clusters;
 }
 
-static int launch_evolve(vqemps_ctx *ctx, const double *theta_dev, int B, cudaStream_t st) {
+// The gate chain.
+static int launch_chain(vqemps_ctx *ctx, const double *theta_dev, int B, cudaStream_t st) {
   ctx->ladder_B = 0;
   EvolveParams ep{};
   ep.gates = ctx->d_gates;
@@ -1173,6 +1180,27 @@ static int launch_evolve(vqemps_ctx *ctx, const double *theta_dev, int B, cudaSt
       evolve_kernel<<<B, EVOLVE_THREADS, EvolveSmem::bytes(ctx->n), st>>>(ep);
   }
   CUDA_TRY(ctx, cudaGetLastError());
+  return VQEMPS_OK;
+}
+
+// The exact bond-doubling state replaces the chain where the chain's SVDs discard nothing: only
+// adjacent CX, zero cutoffs, doubled bonds within max_bond, and no chain asked for by name. The
+// states are equal (in another gauge), and so are the per-state failures: the rank guard cannot
+// fire, and an angle that is not finite fails its state in both.
+static bool exact_states_at(const vqemps_ctx *ctx, bool doubling_ok, int doubled_bond) {
+  return doubling_ok && ctx->evolve_pair < 0 && ctx->abs_cut == 0.0 && ctx->rel_cut == 0.0 && doubled_bond <= ctx->max_bond;
+}
+
+static int launch_evolve(vqemps_ctx *ctx, const double *theta_dev, int B, cudaStream_t st) {
+  if (!exact_states_at(ctx, ctx->doubling_ok, ctx->doubled_bond)) return launch_chain(ctx, theta_dev, B, st);
+  CUDA_TRY(ctx, ctx->lad_theta.ensure((size_t)B * std::max(ctx->P, 1)));
+  CUDA_TRY(ctx, cudaMemsetAsync(ctx->status.ptr, 0, sizeof(int32_t) * B, st));
+  exact_sites_kernel<<<dim3(ctx->n, B), EXACT_THREADS, 0, st>>>(ctx->d_events, ctx->d_ev_off, ctx->d_mats, theta_dev, ctx->P,
+                                                                ctx->n, ctx->init0, ctx->init1, ctx->sites.ptr, nullptr,
+                                                                nullptr, ctx->status.ptr, ctx->lad_theta.ptr);
+  CUDA_TRY(ctx, cudaGetLastError());
+  ctx->evolve_launches = 1;
+  ctx->ladder_B = B;
   return VQEMPS_OK;
 }
 
@@ -1796,11 +1824,11 @@ extern "C" int vqemps_copy_sites(vqemps_ctx *ctx, int b, double *sites_host, voi
   if (!ctx || !sites_host || b < 0 || b >= ctx->last_B) return VQEMPS_INVALID;
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = as_stream(stream);
-  if (ctx->ladder_B > 0) {              // the last energies prepared no site tensors: run the gate chain now
+  if (ctx->ladder_B > 0) {              // the last call ran no gate chain: run it now
     if (b >= ctx->ladder_B) return VQEMPS_INVALID;
     const int rc0 = ensure_state_ws(ctx, ctx->ladder_B);
     if (rc0) return rc0;
-    const int rc = launch_evolve(ctx, ctx->lad_theta.ptr, ctx->ladder_B, st);
+    const int rc = launch_chain(ctx, ctx->lad_theta.ptr, ctx->ladder_B, st);
     if (rc) return rc;
   }
   CUDA_TRY(ctx, cudaMemcpyAsync(sites_host, ctx->sites.ptr + (size_t)b * ctx->n * SITE_ELEMS,

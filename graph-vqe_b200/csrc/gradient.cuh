@@ -85,69 +85,88 @@ __device__ __forceinline__ void event_matrix(const SiteEvent &e, const cplx *mat
 }
 
 // ---------------------------------------------------------------------------
-// forward: bond-doubling site tensors, CTA per (site, state)
+// Bond-doubling site tensors, CTA per (site, state). Element (l, p, r) depends only on its own
+// index bits: every CX half reads one bit of l or r (the i-th doubling's bit is the i-th most
+// significant), so each thread carries one (l, r) pair's two amplitudes through the site's
+// events in registers, with no exchange between threads; the gates' matrices are formed first, one
+// thread each. Bound: the 8 KiB written per site (40 qubits, B = 256: 84 MB) and, for small batches, one
+// sincos and the event loop (about 5 us). As a state preparation it replaces the gate chain's serial SVDs wherever
+// they would not truncate: 64 partitions of 8-48 qubits 1,603 us there.
+// Partition sets: state b belongs to partition st_part[b], whose events lie at ev_off rows of
+// stride n + 1. status (optional, zeroed before): a matrix that is not finite fails the state when
+// a CX follows it on its site. keep (optional): a copy of the angles.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(GSITE_THREADS)
-grad_sites_kernel(const SiteEvent *__restrict__ events, const int32_t *__restrict__ ev_off,
-                  const cplx *__restrict__ mats, const double *__restrict__ theta, int P, int n,
-                  cplx init0, cplx init1, cplx *__restrict__ sites) {
-  __shared__ cplx T0[SITE_ELEMS], T1[SITE_ELEMS];
-  __shared__ cplx M[4];
+constexpr int EXACT_THREADS = 256;
+constexpr int EXACT_EVENTS = 64;      // events staged at a time
+
+__global__ void __launch_bounds__(EXACT_THREADS)
+exact_sites_kernel(const SiteEvent *__restrict__ events, const int32_t *__restrict__ ev_off,
+                   const cplx *__restrict__ mats, const double *__restrict__ theta, int P, int n, cplx init0, cplx init1,
+                   cplx *__restrict__ sites, const int32_t *__restrict__ st_part, const int32_t *__restrict__ part_n,
+                   int32_t *__restrict__ status, double *__restrict__ keep) {
+  __shared__ cplx M[EXACT_EVENTS][4];
+  __shared__ int32_t kind[EXACT_EVENTS];
   const int q = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+  const int part = st_part ? st_part[b] : 0;
+  if (st_part && q >= part_n[part]) return;
   const double *theta_b = theta + (size_t)b * P;
-  for (int e = tid; e < SITE_ELEMS; e += GSITE_THREADS)
-    T0[e] = e == 0 ? init0 : (e == CHI ? init1 : cmake(0, 0));
-  int dl = 1, dr = 1;
-  cplx *cur = T0, *nxt = T1;
-  __syncthreads();
-  for (int k = ev_off[q]; k < ev_off[q + 1]; ++k) {
-    const SiteEvent ev = events[k];
-    if (ev.kind == EV_ONE) {
-      if (tid == 0) {
-        cplx dm[4];
-        event_matrix(ev, mats, theta_b, M, dm);
-      }
-      __syncthreads();
-      for (int e = tid; e < CHI * CHI; e += GSITE_THREADS) {
-        const int l = e >> 4, r = e & 15;
-        const cplx a0 = cur[(l * 2 + 0) * CHI + r], a1 = cur[(l * 2 + 1) * CHI + r];
-        cur[(l * 2 + 0) * CHI + r] = cadd(cmul(M[0], a0), cmul(M[1], a1));
-        cur[(l * 2 + 1) * CHI + r] = cadd(cmul(M[2], a0), cmul(M[3], a1));
-      }
-    } else if (ev.kind == EV_CXL) {
-      // new[a][i][b*2+s]: control left -> A[a][i][b] delta_{is}; target left -> A[a][i^s][b]
-      for (int e = tid; e < SITE_ELEMS; e += GSITE_THREADS) {
-        const int a = e >> 5, i = (e >> 4) & 1, col = e & 15;
-        const int bb = col >> 1, s = col & 1;
-        cplx v = cmake(0, 0);
-        if (bb < dr) {
-          if (ev.ctrl_left) v = (i == s) ? cur[(a * 2 + i) * CHI + bb] : cmake(0, 0);
-          else v = cur[(a * 2 + (i ^ s)) * CHI + bb];
+  if (keep != nullptr && q == 0)
+    for (int i = tid; i < P; i += EXACT_THREADS) keep[(size_t)b * P + i] = theta_b[i];
+  const int32_t *off = ev_off + (size_t)part * (n + 1);
+  const int k0 = off[q], k1 = off[q + 1];
+  const int l = tid >> 4, r = tid & 15;
+  // number of doublings on either side and the last of them
+  int nl = 0, nr = 0, last = -1;
+  for (int k = k0; k < k1; ++k) {
+    const int kd = events[k].kind;
+    nl += kd == EV_CXR;
+    nr += kd == EV_CXL;
+    if (kd != EV_ONE) last = k;
+  }
+  cplx a0 = init0, a1 = init1;
+  int il = nl, ir = nr;               // bits still to be read
+  for (int base = k0; base < k1; base += EXACT_EVENTS) {
+    const int cnt = min(EXACT_EVENTS, k1 - base);
+    __syncthreads();
+    if (tid < cnt) {
+      const SiteEvent ev = events[base + tid];
+      kind[tid] = ev.kind == EV_ONE ? 0 : (ev.kind == EV_CXL ? 1 : 3) + (ev.ctrl_left ? 1 : 0);
+      if (ev.kind == EV_ONE) {
+        cplx m[4], dm[4];
+        event_matrix(ev, mats, theta_b, m, dm);
+        bool ok = true;
+        for (int i = 0; i < 4; ++i) {
+          M[tid][i] = m[i];
+          ok = ok && isfinite(m[i].x) && isfinite(m[i].y);
         }
-        nxt[e] = v;
+        if (!ok && base + tid < last && status != nullptr) status[b] = ST_NONFINITE;
       }
-      dr *= 2;
-      cplx *t = cur; cur = nxt; nxt = t;
-    } else {
-      // new[b*2+s][j][r]: control left (site is target) -> B[b][j^s][r];
-      //                   control right (site is control) -> B[b][j][r] delta_{js}
-      for (int e = tid; e < SITE_ELEMS; e += GSITE_THREADS) {
-        const int row = e >> 5, j = (e >> 4) & 1, r = e & 15;
-        const int bb = row >> 1, s = row & 1;
-        cplx v = cmake(0, 0);
-        if (bb < dl) {
-          if (ev.ctrl_left) v = cur[(bb * 2 + (j ^ s)) * CHI + r];
-          else v = (j == s) ? cur[(bb * 2 + j) * CHI + r] : cmake(0, 0);
-        }
-        nxt[e] = v;
-      }
-      dl *= 2;
-      cplx *t = cur; cur = nxt; nxt = t;
     }
     __syncthreads();
+    for (int k = 0; k < cnt; ++k) {
+      const int kd = kind[k];
+      if (kd == 0) {
+        const cplx b0 = cadd(cmul(M[k][0], a0), cmul(M[k][1], a1));
+        a1 = cadd(cmul(M[k][2], a0), cmul(M[k][3], a1));
+        a0 = b0;
+        continue;
+      }
+      // left half (1 target, 2 control), right half (3 control, 4 target): control copies the bit, target flips by it
+      const int bit = kd <= 2 ? (r >> --ir) & 1 : (l >> --il) & 1;
+      if (kd == 2 || kd == 3) {
+        if (bit) a0 = cmake(0, 0);
+        else a1 = cmake(0, 0);
+      } else if (bit) {
+        const cplx t = a0;
+        a0 = a1;
+        a1 = t;
+      }
+    }
   }
+  if ((l >> nl) != 0 || (r >> nr) != 0) a0 = a1 = cmake(0, 0);
   cplx *dst = sites + ((size_t)b * n + q) * SITE_ELEMS;
-  for (int e = tid; e < SITE_ELEMS; e += GSITE_THREADS) dst[e] = cur[e];
+  dst[(l * 2 + 0) * CHI + r] = a0;
+  dst[(l * 2 + 1) * CHI + r] = a1;
 }
 
 // ---------------------------------------------------------------------------

@@ -234,7 +234,9 @@ class Engine:
         order) or 'auto' (default: quad for a circuit of real gates while all its
         clusters fit the GPU at once, else pair while the batch has at most two
         states per SM, else chain). All give the same states bit for bit. With
-        'auto', energies of ladder circuits run no chain at all (include/vqemps.h)."""
+        'auto', circuits that the chain would not truncate are prepared as exact
+        bond-doubling states instead, and energies of ladder circuits prepare no
+        site tensors at all (include/vqemps.h)."""
         check(self.ctx, self.lib.vqemps_set_evolve_mode(
             self.ctx, {"chain": 0, "pair": 1, "quad": 2, "auto": -1}[mode]), "set_evolve_mode")
 

@@ -240,15 +240,19 @@ int vqemps_set_split_mode(vqemps_ctx *ctx, int mode);
  * CTA per state in program order; -1 (default) uses 2 for a circuit of real gates
  * while all clusters of four fit the GPU at once and the four-gate schedule is
  * shorter, else 1 while the batch has at most twice as many states as the GPU has
- * SMs, else 0. All give the same states bit for bit.
- * Energies of ladder circuits (vqemps_set_level_variant) run no chain at -1. */
+ * SMs, else 0. All give the same states bit for bit. At -1 the chain runs only
+ * where it may truncate: a circuit whose two-qubit gates are adjacent CX, at zero
+ * cutoffs and with 2^(CX on a bond) <= max_bond, is prepared as the exact
+ * bond-doubling state instead (the same state in another gauge), and energies of
+ * ladder circuits (vqemps_set_level_variant) prepare no site tensors at all. */
 int vqemps_set_evolve_mode(vqemps_ctx *ctx, int mode);
 
 /* Copy the site tensors of state b of the last batched call to the host:
  * n * 16 * 2 * 16 complex (re, im) pairs, site s at offset s * 1024 doubles,
  * element (l, p, r) at ((l * 2 + p) * 16 + r), zero padded beyond the bond dims.
- * Used to check the prepared state against the oracle (synchronises). After
- * energies of a ladder circuit the gate chain runs here, on the call's angles. */
+ * Used to check the prepared state against the oracle (synchronises). After a
+ * call that ran no gate chain (vqemps_set_evolve_mode) the chain runs here, on
+ * that call's angles. */
 int vqemps_copy_sites(vqemps_ctx *ctx, int b, double *sites_host, void *stream);
 
 /* Partition sets: K independent circuits of uneven width, parameter count and
