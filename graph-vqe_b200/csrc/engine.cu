@@ -1220,7 +1220,7 @@ static int launch_right(vqemps_ctx *ctx, Hamiltonian *h, int B, cudaStream_t st,
                                                       ctx->status.ptr, h ? ctx->leafval.ptr : nullptr, nleaf,
                                                       h ? h->e_identity_leaf() : -1, ctx->right_real.ptr,
                                                       panels ? ctx->panels.ptr : nullptr,
-                                                      panels_t ? ctx->panels_t.ptr : nullptr);
+                                                      panels_t ? ctx->panels_t.ptr : nullptr, nullptr, nullptr, nullptr);
     ctx->right_real_fresh = true;
     ctx->panels_fresh = panels;
     ctx->panels_t_fresh = panels_t;

@@ -181,18 +181,27 @@ __device__ __forceinline__ void class_tiles_real_iz(const double *A, const doubl
 
 // One trie level for B states (uniform batch: state blockIdx.y, groups
 // interleaved over the grid, groups_per_warp each), environments as real parts.
-// Five CTAs per SM (96 registers, 35 KB of shared memory each): measured 3 %
-// faster at 40 qubits / B = 256 than four (120 registers).
-__global__ void __launch_bounds__(RL_WARPS * 32, 5)
-level_real_pf_kernel(LevelParams p, int groups_per_warp) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+// PARTS: a partition set's work list instead (one item per CTA), and a leaf's products rounded before
+// they are added, as the complex kernel rounds them beside its exact-zero imaginary products: every
+// environment and value has the complex three-product kernel's bits (its other terms are
+// exact zeros here, and Re = k1 - 0, Im = k1 - k1).
+template <bool PARTS>
+__device__ __forceinline__ void level_real_body(const LevelParams &p, int groups_per_warp, unsigned char *smem_raw) {
   LevelRealSmem &sm = *reinterpret_cast<LevelRealSmem *>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = p.flip ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
-  const int stride = gridDim.x * RL_WARPS;
-  const int first = blockIdx.x * RL_WARPS + warp;
-  int count = 0;
-  if (first < p.ngroups) count = min(groups_per_warp, (p.ngroups - first + stride - 1) / stride);
+  int b, stride, first, count = 0;
+  if constexpr (PARTS) {
+    const int32_t *w = p.work + 3 * blockIdx.x;
+    b = w[0];
+    stride = RL_WARPS;
+    first = w[1] + warp;
+    if (warp < w[2]) count = (w[2] - warp + RL_WARPS - 1) / RL_WARPS;
+  } else {
+    b = p.flip ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
+    stride = gridDim.x * RL_WARPS;
+    first = blockIdx.x * RL_WARPS + warp;
+    if (first < p.ngroups) count = min(groups_per_warp, (p.ngroups - first + stride - 1) / stride);
+  }
   if (threadIdx.x == 0) {
     mbar_init(&sm.bar_cta, 1);
     for (int w = 0; w < RL_WARPS; ++w) mbar_init(&sm.bar_warp[w], 1);
@@ -338,9 +347,17 @@ level_real_pf_kernel(LevelParams p, int groups_per_warp) {
 #pragma unroll
               for (int ct = rt; ct < 2; ++ct)
 #pragma unroll
-                for (int j = 0; j < 2; ++j) v += out[rt][ct][j] * R[rl_swz(rt * 8 + g, ct * 8 + 2 * t + j)];
+                for (int j = 0; j < 2; ++j) {
+                  const double r = R[rl_swz(rt * 8 + g, ct * 8 + 2 * t + j)];
+                  if constexpr (PARTS) v = __dadd_rn(v, __dmul_rn(out[rt][ct][j], r));
+                  else v += out[rt][ct][j] * r;
+                }
 #pragma unroll
-            for (int j = 0; j < 2; ++j) v += sc * out[0][1][j] * R[rl_swz(8 + 2 * t + j, g)];
+            for (int j = 0; j < 2; ++j) {
+              const double r = R[rl_swz(8 + 2 * t + j, g)];
+              if constexpr (PARTS) v = __dadd_rn(v, __dmul_rn(out[0][1][j], r));   // sc is 1 where a value counts
+              else v += sc * out[0][1][j] * r;
+            }
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
           }
           if (lane == 0) p.leafval[(size_t)b * p.nleaf_total + node.leaf] = w * v;
@@ -351,6 +368,23 @@ level_real_pf_kernel(LevelParams p, int groups_per_warp) {
     grp = grp_next;
     if (more && lane < grp.nchild) nd = p.nodes[grp.child_begin + lane];
   }
+}
+
+// Five CTAs per SM (96 registers, 35 KB of shared memory each): measured 3 %
+// faster at 40 qubits / B = 256 than four (120 registers).
+__global__ void __launch_bounds__(RL_WARPS * 32, 5)
+level_real_pf_kernel(LevelParams p, int groups_per_warp) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  level_real_body<false>(p, groups_per_warp, smem_raw);
+}
+
+// A partition set of circuits of real gates: one DMMA product where the complex work-list kernel
+// issues three (64 partitions of 8-48 qubits, the 48 levels: 1,935 -> 805 us,
+// the whole call 2,182 -> 918; the levels are short, 17 us of one to two waves each).
+__global__ void __launch_bounds__(RL_WARPS * 32, 5)
+level_real_parts_kernel(LevelParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  level_real_body<true>(p, 0, smem_raw);
 }
 
 // The pair closures of the split evaluation on real-part environments:
@@ -459,20 +493,24 @@ right_env_real_kernel(const cplx *__restrict__ sites, int n, cplx *__restrict__ 
                       cplx *__restrict__ branch, const int32_t *__restrict__ status,
                       double *__restrict__ leafval, int nleaf_total, int identity_leaf,
                       double *__restrict__ right_real, double *__restrict__ panels,
-                      double *__restrict__ panels_t) {
+                      double *__restrict__ panels_t, const int32_t *__restrict__ st_part,
+                      const int32_t *__restrict__ part_n, const int32_t *__restrict__ part_idleaf) {
   constexpr int AS = 2 * CHI + 1;
   __shared__ double A[CHI * AS];
   __shared__ double R[ENV_ELEMS];
   __shared__ double T[2 * ENV_ELEMS];
   const int b = blockIdx.x, tid = threadIdx.x;
+  // partition sets: n is the widest partition (the stride), nb this state's width
+  const int nb = st_part ? part_n[st_part[b]] : n;
+  if (st_part) identity_leaf = part_idleaf[st_part[b]];
   const cplx *sb = sites + (size_t)b * n * SITE_ELEMS;
   cplx *rb = right + (size_t)b * (n + 1) * ENV_ELEMS;
   double *rr = right_real + (size_t)b * (n + 1) * ENV_ELEMS;
   cplx *mbase = branch ? branch + (size_t)b * n * 2 * ENV_ELEMS : nullptr;
   R[tid] = tid == 0 ? 1.0 : 0.0;
-  rb[(size_t)n * ENV_ELEMS + tid] = cmake(R[tid], 0.0);
-  rr[(size_t)n * ENV_ELEMS + rl_swz(tid >> 4, tid & 15)] = R[tid];
-  for (int s = n - 1; s >= 0; --s) {
+  rb[(size_t)nb * ENV_ELEMS + tid] = cmake(R[tid], 0.0);
+  rr[(size_t)nb * ENV_ELEMS + rl_swz(tid >> 4, tid & 15)] = R[tid];
+  for (int s = nb - 1; s >= 0; --s) {
     for (int e = tid; e < SITE_ELEMS; e += RIGHT_THREADS) A[(e >> 5) * AS + (e & 31)] = sb[(size_t)s * SITE_ELEMS + e].x;
     __syncthreads();
     if (panels != nullptr) {

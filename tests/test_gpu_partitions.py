@@ -175,3 +175,26 @@ def test_uneven_64_partitions_full_size(vq):
         assert np.all(np.abs(es - e) <= 6 * bound)
         counts = vq.counts(bits, ps.n_max, 0)
         assert sum(counts.values()) == shots
+
+
+@pytest.mark.parametrize("order", ["msb", "qubit"])
+def test_real_partition_sets_equal_the_pinned_engine_bitwise(vq, order):
+    """Sets whose circuits are all of real gates run their levels in real arithmetic: the same bits as
+    the complex kernel, which drops products with exact zeros only. Widths from 2 to past a bond's
+    saturation, Hamiltonians from one word to several work items per level, an odd number of Y's."""
+    rng = np.random.default_rng(17)
+    parts = []
+    for k, (n, T, L) in enumerate([(2, 3, 1), (3, 1, 2), (9, 40, 4), (17, 900, 4), (33, 130, 3)]):
+        spec = O.hardware_efficient_spec(n, L, ("ry",), ("linear", "reverse_linear")[k % 2])
+        words, coeffs = random_hamiltonian(rng, n, T, 4)
+        if n > 3:
+            words[1], words[2] = "Y" + "I" * (n - 1), "IYXY" + "I" * (n - 4)
+        parts.append((spec, words, np.asarray(coeffs), rng.uniform(-np.pi, np.pi, spec["count"])))
+    eng = vq.Engine(0, 16)
+    ps = _load(vq, eng, parts, order)
+    e, pt = eng.partition_energy(ps, ps.pack_theta([p[3] for p in parts], device=eng.device), per_term=True)
+    for k, (spec, words, coeffs, x) in enumerate(parts):
+        se, sh = _single(vq, spec, words, coeffs, order)
+        e1, pt1 = se.energy(sh, x, per_term=True)
+        assert e1.item() == e[k].item()
+        assert np.array_equal(pt1.cpu().numpy()[0], pt[k, :len(words)].cpu().numpy())
