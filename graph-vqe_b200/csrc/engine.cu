@@ -347,6 +347,7 @@ struct vqemps_ctx {
   DevBuf<uint64_t> bits, seeds;
   DevBuf<int32_t> zsum;
   DevBuf<cplx> branch;
+  DevBuf<double> sample_thr, sample_vec;   // shot prefixes
   DevBuf<double> analytic_stage;
   DevBuf<cplx> grad_sites, grad_envs, grad_seg, grad_bar0, grad_bar1, grad_sitebar, grad_partial, grad_leafsum;
   // split gradient: transposed sites, suffix environments (all levels), suffix
