@@ -356,7 +356,7 @@ struct vqemps_ctx {
   // second stream) and the left sweep's F at the cut
   DevBuf<cplx> grad_sites_t, grad_senv, grad_sbar0, grad_sbar1, grad_rootbar, grad_partial_s, grad_fstate;
   DevBuf<double> grad_stage;
-  DevBuf<double> lad_coef, lad_poison, lad_envp, lad_envs, lad_theta;
+  DevBuf<double> lad_coef, lad_const, lad_poison, lad_envp, lad_envs, lad_theta;
   DevBuf<double> lad_cotp, lad_cots, lad_part, lad_sums;   // ladder gradients
   int ladder_list = -1;                 // task list of the ladder kernels, -1: by batch size
   int ladder_launches = 0;              // kernels the last run_ladder launched
@@ -446,8 +446,10 @@ extern "C" int vqemps_create(int device, int max_bond, double abs_cut, double re
                        (int)sizeof(LevelMmaPfSmem));
   cudaFuncSetAttribute(level_mma3_pf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(LevelMmaPfSmem));
-  cudaFuncSetAttribute(ladder_back_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lad_back_smem<true>());
-  cudaFuncSetAttribute(ladder_back_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lad_back_smem<false>());
+  cudaFuncSetAttribute(ladder_back_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lad_back_smem<true>());
+  cudaFuncSetAttribute(ladder_back_kernel<true, LAD_TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lad_back_smem<true>());
+  cudaFuncSetAttribute(ladder_back_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lad_back_smem<false>());
+  cudaFuncSetAttribute(ladder_back_kernel<false, LAD_TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lad_back_smem<false>());
   grad_set_attributes();
   cudaFuncSetAttribute(grad_fwd_level_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(GradFwdMmaSmem));

@@ -31,8 +31,9 @@
 // there are eight). S1-S3 need no exchange; S4 and SF exchange digit 4 with one shuffle per
 // component, and between identity codes not even that. A warp walks a whole path of trie
 // nodes without touching memory except for the site's rotations (22 or 39 numbers) and the
-// environments that several paths or a closure need. Those lie in global memory as
-// [slot][digit 4][digits 1-3][state], so that eight states fill the 32-byte sectors.
+// environments that several paths or a closure need. Those lie in global memory in 16-byte pairs of
+// components (see lad_at): eight states side by side where the batch has them, so that a warp's access is
+// full 128-byte lines, else one block per state.
 #pragma once
 #include "common.cuh"
 #include "evolve.cuh"
@@ -64,7 +65,9 @@ struct LadCoefParams {
   double *poison;          // B: 0, or NaN when an angle is not finite
   double *leafval;         // B x nleaf: leaf 0 the norm, leaf 1 zero
   int nleaf;
+  double *consts;          // LAD_CONSTS environments: the prefix and the suffix boundary, zero (or null)
 };
+constexpr int LAD_CONSTS = 3;
 
 __device__ __forceinline__ void mul2(const cplx *a, const cplx *b, cplx *o) {
   o[0] = cadd(cmul(a[0], b[0]), cmul(a[1], b[2]));
@@ -89,6 +92,93 @@ __device__ __forceinline__ void bloch(const cplx *u, double *o) {
   o[8] = 0.5 * ((cabs2(u[0]) - cabs2(u[1])) - (cabs2(u[2]) - cabs2(u[3])));
 }
 
+// ---- a quad's components ------------------------------------------------------
+// Lane q of a quad holds the components with digit 4 = q.
+//
+// Complex amplitudes: x[d1 + 4 d2 + 16 d3], all 64.
+//
+// Real amplitudes: only components of one Y parity are nonzero, so the lane's class c (parity of
+// Y among digits 1-3: the word's parity so far, the other one on lane Y) selects 36 (c = 0) or 28
+// (c = 1) of the 64. They are grouped by g = d1 + 4 d2: a group whose own Y parity equals c has
+// d3 in {I, X, Z}, the others only d3 = Y. x[g] holds the group's X or Y component, x[16 + 2 m] and
+// x[17 + 2 m] the I and Z components of the m-th group of parity c (10 or 6 of them; the rest of the
+// 36 slots is zero). With these slots S4 and SF, which mix lanes of different classes, are the same
+// instructions for every lane; only S1-S3 are written per class.
+constexpr int LAD_XR = 36, LAD_XC = 64;
+template <bool REAL> __host__ __device__ constexpr int lad_lane_comps() { return REAL ? LAD_XR : LAD_XC; }
+
+template <int I> struct LadInt { static constexpr int v = I; };
+template <int N, typename F>
+__device__ __forceinline__ void lad_for(F &&f) {
+  if constexpr (N > 0) {
+    lad_for<N - 1>(f);
+    f(LadInt<N - 1>{});
+  }
+}
+__host__ __device__ constexpr int lad_gpar(int g) { return ((g & 3) == 2) ^ ((g >> 2) == 2) ? 1 : 0; }
+__host__ __device__ constexpr int lad_rank(int g, int par) {   // groups of that parity before g
+  int m = 0;
+  for (int i = 0; i < g; ++i) m += lad_gpar(i) == par;
+  return m;
+}
+// slot of component (d1, d2, d3) in class c (which must contain it)
+template <int C, int D1, int D2, int D3>
+__device__ constexpr int lad_slot() {
+  constexpr int g = D1 + 4 * D2;
+  return (D3 == 1 || D3 == 2) ? g : 16 + 2 * lad_rank(g, C) + (D3 == 3 ? 1 : 0);
+}
+
+// Environments in memory, offsets between a lane's pairs known to the compiler whatever the batch size:
+//   W = 8: [slot][tile of 8 states][digit 4][pair][state][2], a warp's access to a digit is one 128-byte line;
+//   W = 1: [slot][state][pair][digit 4: I Z X Y][2], a quad's access is 64 contiguous bytes, and steps that
+//          keep only I and Z still move whole sectors.
+// Batches of a multiple of 8 take W = 8: others would straddle tiles (45 complex states 110 us with W = 1, 118 with
+// W = 8). Against
+// 8-byte accesses at a run-time stride: LAYOUTMEASURED
+constexpr int LAD_TILE = 8;
+__host__ __device__ constexpr bool lad_tiled(int B) { return B > 0 && B % LAD_TILE == 0; }
+// offset of state b's environment from its slot's start (slots are B x 4 N apart)
+template <int W, int N>
+__device__ __forceinline__ size_t lad_state(int b) {
+  return W == 1 ? (size_t)b * (4 * N) : (size_t)(b / W) * (W * 4 * N) + 2 * (b % W);
+}
+// this lane's pairs of an environment (at lad_state), lad_stride pairs apart
+template <int W, int N>
+__device__ __forceinline__ const double2 *lad_at(const double *env, int role) {
+  const int place = role == 0 ? 0 : (role == 3 ? 1 : role + 1);
+  return reinterpret_cast<const double2 *>(env) + (W == 1 ? place : place * (N / 2) * W);
+}
+template <int W> __host__ __device__ constexpr int lad_stride() { return W == 1 ? 4 : W; }
+// A lane's share of an environment; real environments of class 1 carry zeros in the slots they do not use.
+template <int W, int N>
+__device__ __forceinline__ void lad_get(double (&x)[N], const double *env, int role) {
+  const double2 *src = lad_at<W, N>(env, role);
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    const double2 v = src[lad_stride<W>() * i];
+    x[2 * i] = v.x;
+    x[2 * i + 1] = v.y;
+  }
+}
+template <int W, int N>
+__device__ __forceinline__ void lad_put(const double (&x)[N], double *env, int role) {
+  double2 *dst = const_cast<double2 *>(lad_at<W, N>(env, role));
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) dst[lad_stride<W>() * i] = make_double2(x[2 * i], x[2 * i + 1]);
+}
+// boundary: prefix |0> in every digit (I = Z = 1), suffix all ones (I = X = 1)
+template <bool REAL>
+__device__ __forceinline__ void lad_boundary(double (&x)[lad_lane_comps<REAL>()], int role, bool suffix) {
+  const int other = suffix ? 1 : 3;
+  auto in = [&](int d) { return d == 0 || d == other; };
+  lad_for<64>([&](auto J) {
+    constexpr int j = decltype(J)::v, d1 = j & 3, d2 = (j >> 2) & 3, d3 = j >> 4;
+    const double v = in(d1) && in(d2) && in(d3) && in(role) ? 1.0 : 0.0;
+    if constexpr (!REAL) x[j] = v;
+    else if constexpr (((d1 == 2) ^ (d2 == 2) ^ (d3 == 2)) == 0) x[lad_slot<0, d1, d2, d3>()] = v;
+  });
+}
+
 // Rotations of every site and layer, one CTA per state. A layer before the site's last CX with
 // an angle that is not finite fails the state (as the SVD chain's nonfinite check does); such
 // an angle in the last layer only makes the values NaN.
@@ -102,6 +192,20 @@ ladder_coef_kernel(LadCoefParams p) {
   constexpr int NC = REAL ? LAD_REAL_COEFS : LAD_COEFS;
   const double r2 = 0.70710678118654752440;
   const cplx had[4] = {cmake(r2, 0), cmake(r2, 0), cmake(r2, 0), cmake(-r2, 0)};
+  if (p.consts != nullptr && b == 0) {
+    constexpr int NX = lad_lane_comps<REAL>();
+    const bool tiled = lad_tiled(B);
+    const size_t env = (size_t)(tiled ? LAD_TILE : 1) * (4 * NX);
+    if (tid < 4 * LAD_CONSTS) {
+      double x[NX];
+      lad_boundary<REAL>(x, tid & 3, (tid >> 2) == 1);
+      if (tid >= 8)
+        for (double &v : x) v = 0.0;
+      double *dst = p.consts + (tid >> 2) * env;
+      if (tiled) lad_put<LAD_TILE>(x, dst, tid & 3);
+      else lad_put<1>(x, dst, tid & 3);
+    }
+  }
   int bad = 0;
   const int pad = LAD_MAX_LAYERS - p.layers;        // leading layers without a CX
   for (int it = tid; it < p.n * 5; it += 256) {
@@ -161,42 +265,6 @@ ladder_coef_kernel(LadCoefParams p) {
     p.leafval[(size_t)b * p.nleaf] = 1.0 + ps;
     p.leafval[(size_t)b * p.nleaf + 1] = ps;
   }
-}
-
-// ---- a quad's components ------------------------------------------------------
-// Lane q of a quad holds the components with digit 4 = q.
-//
-// Complex amplitudes: x[d1 + 4 d2 + 16 d3], all 64.
-//
-// Real amplitudes: only components of one Y parity are nonzero, so the lane's class c (parity of
-// Y among digits 1-3: the word's parity so far, the other one on lane Y) selects 36 (c = 0) or 28
-// (c = 1) of the 64. They are grouped by g = d1 + 4 d2: a group whose own Y parity equals c has
-// d3 in {I, X, Z}, the others only d3 = Y. x[g] holds the group's X or Y component, x[16 + 2 m] and
-// x[17 + 2 m] the I and Z components of the m-th group of parity c (10 or 6 of them; the rest of the
-// 36 slots is zero). With these slots S4 and SF, which mix lanes of different classes, are the same
-// instructions for every lane; only S1-S3 are written per class.
-constexpr int LAD_XR = 36, LAD_XC = 64;
-template <bool REAL> __host__ __device__ constexpr int lad_lane_comps() { return REAL ? LAD_XR : LAD_XC; }
-
-template <int I> struct LadInt { static constexpr int v = I; };
-template <int N, typename F>
-__device__ __forceinline__ void lad_for(F &&f) {
-  if constexpr (N > 0) {
-    lad_for<N - 1>(f);
-    f(LadInt<N - 1>{});
-  }
-}
-__host__ __device__ constexpr int lad_gpar(int g) { return ((g & 3) == 2) ^ ((g >> 2) == 2) ? 1 : 0; }
-__host__ __device__ constexpr int lad_rank(int g, int par) {   // groups of that parity before g
-  int m = 0;
-  for (int i = 0; i < g; ++i) m += lad_gpar(i) == par;
-  return m;
-}
-// slot of component (d1, d2, d3) in class c (which must contain it)
-template <int C, int D1, int D2, int D3>
-__device__ constexpr int lad_slot() {
-  constexpr int g = D1 + 4 * D2;
-  return (D3 == 1 || D3 == 2) ? g : 16 + 2 * lad_rank(g, C) + (D3 == 3 ? 1 : 0);
 }
 
 // Rotations of one site (a row of LadCoefParams::coef in shared memory).
@@ -500,7 +568,7 @@ struct LadPathParams {
   const uint32_t *steps;
   const int32_t *slots;
   const double *coef;
-  double *envp, *envs;   // prefix / suffix slots [slot][4 x 36 or 4 x 64][B]
+  double *envp, *envs;   // prefix / suffix environments (lad_at)
   int npre, ntasks;      // tasks 0 .. npre - 1 prefix, npre .. ntasks - 1 suffix
   int B;
 };
@@ -515,10 +583,10 @@ __device__ __forceinline__ void lad_cp16(void *dst, const void *src) {
 // environments, another one about 360 and 72 shuffles) and, for small batches, the latency of one
 // warp's step (1-2 us). Real environments take 72 registers, so four CTAs of four warps fit an SM;
 // complex ones take 128 and two CTAs fit. Measured (B200), whole energy call, gate chain + 16 x 16
-// transfer products -> this: 40 qubits, 5,000 words, B = 256: 5,504 -> 769 us (FP64 pipe 40 % busy, issue 53 %);
+// transfer products -> this: 40 qubits, 5,000 words, B = 256: 5,504 -> 732 us (FP64 pipe 40 % busy, issue 53 %);
 // B = 3: 1,082 -> 62 us; 96 qubits, 40,000 words, B = 2: 3,039 -> 139 us; complex, 27 qubits, 1,300 words,
 // B = 45: 1,191 -> 113 us; error against 64-bit values 1e-13 -> 3e-15 (no SVD in between).
-template <bool REAL>
+template <bool REAL, int W>
 __global__ void __launch_bounds__(LAD_THREADS, REAL ? 4 : 2)
 ladder_path_kernel(LadPathParams p) {
   constexpr int NC = REAL ? LAD_REAL_COEFS : LAD_COEFS;
@@ -558,32 +626,20 @@ ladder_path_kernel(LadPathParams p) {
   stage(0, w0);
   stage(1, w1);
   stage(2, w2);
-  double *env = (suffix ? p.envs : p.envp) + b;
+  double *env = (suffix ? p.envs : p.envp) + lad_state<W, NX>(b);
+  const size_t slot_size = (size_t)B * (4 * NX);
   double x[NX];
   int swaps = 0;                                             // real: lanes' roles (lad_role)
-  // real environments of class 1 leave the last eight slots unused
-  auto store = [&](int role, int par, bool lanes_xy) {
+  int slot = live ? *slots : 0;                              // the next one: read ahead, the lists end with a spare entry
+  auto advance = [&] { slot = *++slots; };
+  auto store = [&](int role, bool lanes_xy) {
     if (!lanes_xy && role != 0 && role != 3) return;
-    double *dst = env + ((size_t)(*slots) * (4 * NX) + role * NX) * B;
-    const bool all = !REAL || !(par ^ (role == 2));
-#pragma unroll
-    for (int j = 0; j < NX; ++j)
-      if (j < 28 || all) dst[(size_t)j * B] = x[j];
+    lad_put<W>(x, env + slot * slot_size, role);
   };
-  {
-    // boundary: prefix |0> in every digit (I = Z = 1), suffix all ones (I = X = 1)
-    const int other = suffix ? 1 : 3;
-    auto in = [&](int d) { return d == 0 || d == other; };
-    lad_for<64>([&](auto J) {
-      constexpr int j = decltype(J)::v, d1 = j & 3, d2 = (j >> 2) & 3, d3 = j >> 4;
-      const double v = in(d1) && in(d2) && in(d3) && in(q) ? 1.0 : 0.0;
-      if constexpr (!REAL) x[j] = v;
-      else if constexpr (((d1 == 2) ^ (d2 == 2) ^ (d3 == 2)) == 0) x[lad_slot<0, d1, d2, d3>()] = v;
-    });
-    if (live && (task.flags & 8)) {
-      store(q, 0, suffix);
-      ++slots;
-    }
+  lad_boundary<REAL>(x, q, suffix);
+  if (live && (task.flags & 8)) {
+    store(q, suffix);
+    advance();
   }
   int longest = task.nsteps;
   for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(LAD_FULL, longest, o));
@@ -600,12 +656,13 @@ ladder_path_kernel(LadPathParams p) {
     stage(t + 3, w2);
     if (w & 32) {
       swaps = 0;
-      const double *src = env + ((size_t)(*slots) * (4 * NX) + q * NX) * B;
-      ++slots;
-      const bool set = xy || q == 0 || q == 3;
-      const bool all = !REAL || !(par ^ (q == 2));
+      if (xy || q == 0 || q == 3) {
+        lad_get<W>(x, env + slot * slot_size, q);
+      } else {
 #pragma unroll
-      for (int j = 0; j < NX; ++j) x[j] = (set && (j < 28 || all)) ? src[(size_t)j * B] : 0.0;
+        for (int j = 0; j < NX; ++j) x[j] = 0.0;
+      }
+      advance();
     }
     asm volatile("cp.async.wait_group 3;\n" ::);
     __syncwarp();
@@ -641,8 +698,8 @@ ladder_path_kernel(LadPathParams p) {
         }
         __syncwarp();
         if (on && (w & 4)) {
-          store(role, par, (w & 8) != 0);
-          ++slots;
+          store(role, (w & 8) != 0);
+          advance();
         }
       } else {
         int role = lad_role(q, swaps);
@@ -668,8 +725,8 @@ ladder_path_kernel(LadPathParams p) {
         par ^= (code == 2);
         role = lad_role(q, swaps);
         if (on && (w & 4)) {
-          store(role, par, code != 0);
-          ++slots;
+          store(role, code != 0);
+          advance();
         }
       }
     } else {
@@ -690,8 +747,8 @@ ladder_path_kernel(LadPathParams p) {
         lad_skc<1, 4, 16>(x, lad_rot<false>(c, 0, -1.0));
         lad_s1c(x, c[0], -c[1], c[2]);
         if (on && (w & 4)) {
-          store(q, 0, (w & 8) != 0);
-          ++slots;
+          store(q, (w & 8) != 0);
+          advance();
         }
       } else {
         lad_s1c(x, c[0], c[1], c[2]);
@@ -708,8 +765,8 @@ ladder_path_kernel(LadPathParams p) {
           for (int j = 0; j < NX; ++j) x[j] = 0.0;
         }
         if (on && (w & 4)) {
-          store(q, 0, code != 0);
-          ++slots;
+          store(q, code != 0);
+          advance();
         }
       }
     }
@@ -722,10 +779,10 @@ ladder_path_kernel(LadPathParams p) {
 // lanes per (word, state) as the paths, every sum in the same order whatever the batch size.
 struct LadPair {
   int32_t pslot, sslot, leaf;
-  int32_t flags;    // bit 0 odd Y count of the prefix, bit 1 lanes X and Y count (prefix ends with X, Y or Z)
+  int32_t flags;    // bit 1 lanes X and Y count (prefix ends with X, Y or Z)
 };
 
-template <bool REAL>
+template <bool REAL, int W>
 __global__ void __launch_bounds__(256)
 ladder_close_kernel(const double *__restrict__ envp, const double *__restrict__ envs, const LadPair *__restrict__ pairs,
                     int npairs, int B, const int32_t *__restrict__ status, const double *__restrict__ poison,
@@ -741,24 +798,14 @@ ladder_close_kernel(const double *__restrict__ envp, const double *__restrict__ 
     pr = pairs[quad / B];
     b = (int)(quad % B);
     if ((pr.flags & 2) || q == 0 || q == 3) {
-      const double *t = envp + ((size_t)pr.pslot * (4 * NX) + q * NX) * B + b;
-      const double *w = envs + ((size_t)pr.sslot * (4 * NX) + q * NX) * B + b;
-      if (REAL) {
-        double t8[28], w8[28];
-#pragma unroll
-        for (int j = 0; j < 28; ++j) {
-          t8[j] = t[(size_t)j * B];
-          w8[j] = w[(size_t)j * B];
-        }
-#pragma unroll
-        for (int j = 0; j < 28; ++j) v = fma(t8[j], w8[j], v);
-        if (((pr.flags & 1) ^ (q == 2 ? 1 : 0)) == 0) {
-#pragma unroll
-          for (int j = 28; j < 36; ++j) v = fma(t[(size_t)j * B], w[(size_t)j * B], v);
-        }
-      } else {
-#pragma unroll 16
-        for (int j = 0; j < 64; ++j) v = fma(t[(size_t)j * B], w[(size_t)j * B], v);
+      const size_t slot_size = (size_t)B * (4 * NX), at = lad_state<W, NX>(b);
+      const double2 *t = lad_at<W, NX>(envp + at + pr.pslot * slot_size, q);
+      const double2 *w = lad_at<W, NX>(envs + at + pr.sslot * slot_size, q);
+#pragma unroll(REAL ? 18 : 16)
+      for (int i = 0; i < NX / 2; ++i) {
+        const double2 a = t[lad_stride<W>() * i], c = w[lad_stride<W>() * i];
+        v = fma(a.x, c.x, v);
+        v = fma(a.y, c.y, v);
       }
     }
   }

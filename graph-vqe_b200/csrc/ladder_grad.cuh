@@ -32,7 +32,8 @@ struct LadClose {
 };
 
 constexpr int LAD_GR = 16;   // nx nz | k = 2, 3, 4: xx xz zx zz | W: x z of the step's code
-constexpr int LAD_GC = 36;   // nx ny nz | k = 2, 3, 4: O row-major | W: x y z of the step's code | unused
+constexpr int LAD_GC = 36;   // nx ny nz | k = 2: O row-major || k = 3 | 3 unused || k = 4 | W: x y z of the step's code
+constexpr int LAD_GROUP = 12;   // complex derivatives are summed and stored twelve at a time, so that few are live
 
 struct LadBackParams {
   const LadTask *tasks;
@@ -42,7 +43,8 @@ struct LadBackParams {
   const LadClose *closers;
   const double *coef;
   const double *envp, *envs;
-  double *cotp, *cots;       // [cotangent][4 x 36 or 4 x 64][B]
+  const double *consts;      // boundaries and zero (LadCoefParams)
+  double *cotp, *cots;       // cotangents, laid out as the environments
   double *part;              // [step][LAD_GR or LAD_GC][B]
   int npre, ntasks, B;
 };
@@ -152,29 +154,37 @@ __device__ __forceinline__ void lad_quad_sums(const double *g, int q, double *ou
   }
 }
 
-template <bool REAL> __host__ __device__ constexpr int lad_back_threads() { return REAL ? 128 : 32; }
+constexpr int LAD_BACK = 32;         // threads: one warp, so that shared memory holds as many as it can
+template <bool REAL> __host__ __device__ constexpr int lad_back_arrays() { return REAL ? 3 * LAD_XR : 5 * LAD_XC; }
 template <bool REAL> __host__ __device__ constexpr size_t lad_back_smem() {
-  return (size_t)(REAL ? 2 * LAD_XR : 5 * LAD_XC) * lad_back_threads<REAL>() * sizeof(double) +
-         (size_t)2 * (lad_back_threads<REAL>() / 4) * (REAL ? LAD_REAL_COEFS : LAD_COEFS) * sizeof(double);
+  return (size_t)(lad_back_arrays<REAL>() * LAD_BACK + 2 * (LAD_BACK / 4) * (REAL ? LAD_REAL_COEFS : LAD_COEFS)) *
+         sizeof(double);
 }
 
-// Bound: FP64 issue and shared memory (about 750 FP64 instructions and 150 shared accesses per step
-// of eight real environments). Real: the carried and the loaded tensor in registers, two chain
-// members in shared memory (74 KB per CTA of four warps, two CTAs per SM). Complex: the carried
-// tensor and four members in shared memory (82 KB per CTA of one warp, two per SM). Measured (B200), whole
-// gradient call, 16 x 16 transfer products -> this: 64 qubits, 20,000 words, B = 32: 20,850 -> 4,490 us;
-// 40 qubits, 5,000 words, B = 1: 1,488 -> 643 us; complex, 21 qubits, 790 words, B = 7: 876 -> 437 us.
-template <bool REAL>
-__global__ void __launch_bounds__(lad_back_threads<REAL>(), 2)
+// Bound: FP64 issue, shared memory and the latencies that seven warps an SM leave (64 qubits, B = 16: FP64 pipe
+// 25 % busy, shared-memory pipe 57 %). Real: the carried and the worked-on tensor in registers; the
+// step's input, which arrives by cp.async one step ahead, and one chain member in shared memory (30 KB a
+// warp); the other member is formed again, which is cheaper than the place that would cost two warps an SM.
+// What the two classes of lanes share, loads and stores, stands outside their branches: the loop has
+// to stay in the instruction cache. Complex: the carried tensor and four members in shared memory (82 KB a
+// warp, two an SM), rotations read where they are used: held for the step they spilled 5 KB a thread.
+// Measured (B200), whole gradient call, 16 x 16 transfer products -> this: 64 qubits, 20,000 words, B = 32:
+// 20,850 -> 3,626 us; 40 qubits, 5,000 words, B = 1: 1,488 -> 437 us; complex, 21 qubits, 790 words, B = 7:
+// 876 -> 322 us.
+template <bool REAL, int W>
+__global__ void __launch_bounds__(LAD_BACK, REAL ? 7 : 2)
 ladder_back_kernel(LadBackParams p) {
   constexpr int NC = REAL ? LAD_REAL_COEFS : LAD_COEFS;
   constexpr int NX = lad_lane_comps<REAL>();
-  constexpr int NT = lad_back_threads<REAL>();
+  constexpr int NT = LAD_BACK;
   constexpr int NG = REAL ? LAD_GR : LAD_GC;
   extern __shared__ __align__(16) double lad_smem[];
-  double *rows = lad_smem + (size_t)(REAL ? 2 * LAD_XR : 5 * LAD_XC) * NT;      // [2][NT / 4][NC]
+  double *rows = lad_smem + (size_t)lad_back_arrays<REAL>() * NT;      // [2][NT / 4][NC]
   const int tid = threadIdx.x, lane = tid & 31, q = lane & 3;
-  auto keep = [&](int arr, int j) -> double & { return lad_smem[(size_t)(arr * NX + j) * NT + tid]; };
+  auto keep = [&](int arr, int j) -> double & { return lad_smem[(size_t)(arr * NX + j) * NT + tid]; };   // complex
+  auto keep2 = [&](int arr, int i) -> double2 & {                                                    // real: pairs
+    return reinterpret_cast<double2 *>(lad_smem)[(size_t)(arr * (NX / 2) + i) * NT + tid];
+  };
   const int B = p.B;
   const long long quad = ((long long)blockIdx.x * NT + tid) >> 2;
   const long long npre_q = (long long)p.npre * B, pre_pad = (npre_q + 7) & ~7LL;
@@ -187,23 +197,48 @@ ladder_back_kernel(LadBackParams p) {
     task = p.tasks[idx / B];
     b = (int)(idx % B);
   }
-  const double *own = (suffix ? p.envs : p.envp) + b, *other = (suffix ? p.envp : p.envs) + b;
-  double *cots = (suffix ? p.cots : p.cotp) + b;
+  constexpr int ENV = W * 4 * NX;                    // of the constants
+  const size_t slot_size = (size_t)B * (4 * NX), at_b = lad_state<W, NX>(b);
+  const double *own = (suffix ? p.envs : p.envp) + at_b, *other = (suffix ? p.envp : p.envs) + at_b;
+  double *cots = (suffix ? p.cots : p.cotp) + at_b;
   int longest = task.nsteps;
   for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(LAD_FULL, longest, o));
   auto word = [&](int i) { return i >= 0 && i < task.nsteps ? p.steps[task.step + i] : 0u; };
-  auto stage = [&](int t, uint32_t w) {
+  auto record = [&](int i) {
+    int4 v = make_int4(-1, -1, -2, 0);
+    if (i >= 0 && i < task.nsteps) v = *reinterpret_cast<const int4 *>(p.back + task.step + i);
+    return LadBack{v.x, v.y, v.z, v.w};
+  };
+  auto flips = [](uint32_t w) { const int code = w & 3; return code == 0 ? 0 : (code == 2 ? 2 : 1); };
+  // the input environment of a step, for this lane's role at that end
+  auto input_at = [&](const LadBack &rec, uint32_t w, int r) {
+    if (!((w & 128) || r == 0 || r == 3)) return p.consts + 2 * ENV;
+    return rec.in < 0 ? p.consts + (suffix ? ENV : 0) : own + rec.in * slot_size;
+  };
+  // rotations (and real inputs) of iteration t's step
+  auto stage = [&](int t, uint32_t w, const LadBack &rec, int r) {
     if (t < task.nsteps) {
       const double *src = p.coef + ((size_t)(w >> 16) * B + b) * NC;
       double *dst = rows + (size_t)((t & 1) * (NT / 4) + (tid >> 2)) * NC;
 #pragma unroll
       for (int i = 0; i < NC / 2; i += 4)
         if (i + q < NC / 2) lad_cp16(dst + 2 * (i + q), src + 2 * (i + q));
+      if constexpr (REAL) {
+        const double2 *in = lad_at<W, NX>(input_at(rec, w, r), r);
+#pragma unroll
+        for (int i = 0; i < NX / 2; ++i) lad_cp16(&keep2(1 + (t & 1), i), in + lad_stride<W>() * i);
+      }
     }
     asm volatile("cp.async.commit_group;\n" ::);
   };
-  uint32_t w_now = word(task.nsteps - 1), w_prev = word(task.nsteps - 2);
-  stage(0, w_now);
+  uint32_t w_now = word(task.nsteps - 1), w_next = word(task.nsteps - 2);
+  LadBack rec_now{}, rec_next{};       // real: read ahead (complex steps have no registers for it)
+  if (REAL) {
+    rec_now = record(task.nsteps - 1);
+    rec_next = record(task.nsteps - 2);
+  }
+  int close_end = live ? p.back[task.step + task.nsteps].close : 0;
+  stage(0, w_now, rec_now, lad_role(q, flips(w_now)));
   double y[NX];                        // the carried cotangent (right end of the step for prefix, left end for suffix)
 #pragma unroll
   for (int j = 0; j < NX; ++j) y[j] = 0.0;
@@ -213,83 +248,81 @@ ladder_back_kernel(LadBackParams p) {
     const int i = task.nsteps - 1 - t;
     const bool on = i >= 0;
     const uint32_t w = w_now;
-    w_now = w_prev;
-    w_prev = word(i - 2);
-    stage(t + 1, w_now);
-    const int code = w & 3;
+    const LadBack rec = REAL ? rec_now : record(i);
+    w_now = w_next;
+    w_next = word(i - 2);
+    if (REAL) {
+      rec_now = rec_next;
+      rec_next = record(i - 2);
+    }
+    const int code = w & 3, flip = flips(w);
+    if (fresh) swaps = 0;
+    stage(t + 1, w_now, rec_now, lad_role(q, (rec.cot_out != -1 ? 0 : swaps ^ flip) ^ flips(w_now)));
     const int par = (w >> 6) & 1;                    // before the task's own step: left end (prefix), right end (suffix)
     const bool xy = (w & 128) != 0;                  // lanes X, Y of the step's input environment
-    LadBack rec{-1, -1, -2, 0};
-    int close_end = 0;
-    if (on) {
-      rec = p.back[task.step + i];
-      close_end = p.back[task.step + i + 1].close;
-    }
-    const int flip = code == 0 ? 0 : (code == 2 ? 2 : 1);
     const int end_par = par ^ (code == 2);           // at the step's result
     // ---- y: carried, collected and the words that close here
     if (fresh) {
-      swaps = 0;
 #pragma unroll
       for (int j = 0; j < NX; ++j) y[j] = 0.0;
     }
     int role = REAL ? lad_role(q, swaps) : q;
     {
       const bool iz = role == 0 || role == 3;
-      const bool all = !REAL || !(end_par ^ (role == 2));
       if (rec.cot_add >= 0) {
-        const double *src = cots + ((size_t)rec.cot_add * (4 * NX) + role * NX) * B;
+        const double2 *src = lad_at<W, NX>(cots + rec.cot_add * slot_size, role);
 #pragma unroll
-        for (int j = 0; j < NX; ++j)
-          if (j < 28 || all) y[j] += src[(size_t)j * B];
+        for (int i = 0; i < NX / 2; ++i) {
+          const double2 v = src[lad_stride<W>() * i];
+          y[2 * i] += v.x;
+          y[2 * i + 1] += v.y;
+        }
       }
+      if (on)
       for (int c = rec.close; c < close_end; ++c) {
         const LadClose cl = p.closers[c];
         if (!(cl.flags & 2) && !iz) continue;
-        const double *src = other + ((size_t)cl.slot * (4 * NX) + role * NX) * B;
+        const double2 *src = lad_at<W, NX>(other + cl.slot * slot_size, role);
 #pragma unroll
-        for (int j = 0; j < NX; ++j)
-          if (j < 28 || all) y[j] = fma(cl.coef, src[(size_t)j * B], y[j]);
+        for (int i = 0; i < NX / 2; ++i) {
+          const double2 v = src[lad_stride<W>() * i];
+          y[2 * i] = fma(cl.coef, v.x, y[2 * i]);
+          y[2 * i + 1] = fma(cl.coef, v.y, y[2 * i + 1]);
+        }
       }
     }
     asm volatile("cp.async.wait_group 1;\n" ::);
     __syncwarp();
     const double *c = rows + (size_t)((t & 1) * (NT / 4) + (tid >> 2)) * NC;
-    double g[NG];
+    double g[REAL ? NG : LAD_GROUP];
+    auto clear = [&] {
 #pragma unroll
-    for (int j = 0; j < NG; ++j) g[j] = 0.0;
-    // the step's input environment, lanes by role r
-    auto input = [&](double (&x)[NX], int r, int rpar) {
-      if (rec.in < 0) {
-        const int o = suffix ? 1 : 3;
-        auto in = [&](int d) { return d == 0 || d == o; };
-        lad_for<64>([&](auto J) {
-          constexpr int j = decltype(J)::v, d1 = j & 3, d2 = (j >> 2) & 3, d3 = j >> 4;
-          const double v = in(d1) && in(d2) && in(d3) && in(r) ? 1.0 : 0.0;
-          if constexpr (!REAL) x[j] = v;
-          else if constexpr (((d1 == 2) ^ (d2 == 2) ^ (d3 == 2)) == 0) x[lad_slot<0, d1, d2, d3>()] = v;
-        });
-        return;
-      }
-      const double *src = own + ((size_t)rec.in * (4 * NX) + r * NX) * B;
-      const bool set = on && (xy || r == 0 || r == 3);
-      const bool all = !REAL || !(rpar ^ (r == 2));
-#pragma unroll
-      for (int j = 0; j < NX; ++j) x[j] = (set && (j < 28 || all)) ? src[(size_t)j * B] : 0.0;
+      for (double &v : g) v = 0.0;
     };
+    clear();
+    // derivatives first .. of this step, summed over the quad
+    auto flush = [&](int first) {
+      constexpr int N = REAL ? NG : LAD_GROUP;
+      double sums[N / 4];
+      lad_quad_sums<N>(g, q, sums);
+      if (on) {
+        double *dst = p.part + ((size_t)(task.step + i) * NG + first + (N / 4) * (2 * (q & 1) + (q >> 1))) * B + b;
+#pragma unroll
+        for (int j = 0; j < N / 4; ++j) dst[(size_t)j * B] = sums[j];
+      }
+    };
+    if (on) close_end = rec.close;
     if constexpr (REAL) {
       double x[NX];
-      const LadRot o2 = lad_rot<true>(c, 0, 1.0), o3 = lad_rot<true>(c, 1, 1.0), o4 = lad_rot<true>(c, 2, 1.0);
       // roles at the left end; SF and its transpose scale a lane by the same factor, set by its role there
       const int lswaps = suffix ? swaps : swaps ^ flip;
       const int lrole = lad_role(q, lswaps), prole = lrole ^ 1;
-      const int rrole = lad_role(q, lswaps ^ flip);
       const int lpar = suffix ? end_par : par;
       const int cls = lpar ^ (lrole == 2);
       const bool iz = lrole == 0 || lrole == 3;
       const int src = (lane & ~3) | lad_role(prole, lswaps);
       const double u = lad_factor(c, code, lrole, 1.0), up = lad_factor(c, code, prole, 1.0);
-      const LadS4 r4 = lad_s4_rows<true>(o4, lrole);
+      const LadS4 r4 = lad_s4_rows<true>(lad_rot<true>(c, 2, 1.0), lrole);
       const bool hi = lrole >= 2;
       const bool left_xy = suffix ? (w & 8) != 0 : xy;                 // lanes X, Y at the left end count
       const bool any = __any_sync(LAD_FULL, on && (code != 0 || left_xy));
@@ -297,25 +330,34 @@ ladder_back_kernel(LadBackParams p) {
       const double s0 = hi ? -r4.sy : r4.sx, s1 = hi ? r4.sy : r4.sx;
       const double ce = cls ? s1 : s0, co = cls ? s0 : s1;
       double ga = 0.0, gb = 0.0, gw = 0.0;
+      auto put = [&] {
+#pragma unroll
+        for (int i = 0; i < NX / 2; ++i) keep2(0, i) = make_double2(x[2 * i], x[2 * i + 1]);
+      };
+      auto get = [&](int arr) {
+#pragma unroll
+        for (int i = 0; i < NX / 2; ++i) {
+          const double2 v = keep2(arr, i);
+          x[2 * i] = v.x;
+          x[2 * i + 1] = v.y;
+        }
+      };
       if (!suffix) {
-        // t -> T1 (kept), T2 (kept), T3
-        input(x, lrole, lpar);
-        if (busy && cls == 0) {
-          lad_s1r<0>(x, c[0], c[1]);
-#pragma unroll
-          for (int j = 0; j < NX; ++j) keep(0, j) = x[j];
-          lad_skr<0, 2>(x, o2);
-#pragma unroll
-          for (int j = 0; j < NX; ++j) keep(1, j) = x[j];
-          lad_skr<0, 3>(x, o3);
-        } else if (busy) {
-          lad_s1r<1>(x, c[0], c[1]);
-#pragma unroll
-          for (int j = 0; j < NX; ++j) keep(0, j) = x[j];
-          lad_skr<1, 2>(x, o2);
-#pragma unroll
-          for (int j = 0; j < NX; ++j) keep(1, j) = x[j];
-          lad_skr<1, 3>(x, o3);
+        // t -> T1, T2 (kept), T3
+        get(1 + (t & 1));
+        if (busy) {
+          const LadRot o2 = lad_rot<true>(c, 0, 1.0);
+          if (cls == 0) {
+            lad_s1r<0>(x, c[0], c[1]);
+            lad_skr<0, 2>(x, o2);
+          } else {
+            lad_s1r<1>(x, c[0], c[1]);
+            lad_skr<1, 2>(x, o2);
+          }
+          put();
+          const LadRot o3 = lad_rot<true>(c, 1, 1.0);
+          if (cls == 0) lad_skr<0, 3>(x, o3);
+          else lad_skr<1, 3>(x, o3);
         }
         __syncwarp();
         // W: products of y with T4 (S4 without the code's factor); S4 and its transpose with their products
@@ -356,59 +398,80 @@ ladder_back_kernel(LadBackParams p) {
         }
         ga *= hi ? u : up;
         gb *= hi ? u : up;
-        if (busy && cls == 0) {
-          lad_gkr<0, 3>(y, [&](int j) { return keep(1, j); }, g[6], g[7], g[8], g[9]);
-          lad_skr<0, 3>(y, o3);
-          lad_gkr<0, 2>(y, [&](int j) { return keep(0, j); }, g[2], g[3], g[4], g[5]);
-          lad_skr<0, 2>(y, o2);
-          input(x, lrole, lpar);
-          lad_g1r<0>(y, [&](int j) { return x[j]; }, g[0], g[1]);
-          lad_s1r<0>(y, c[0], c[1]);
-        } else if (busy) {
-          lad_gkr<1, 3>(y, [&](int j) { return keep(1, j); }, g[6], g[7], g[8], g[9]);
-          lad_skr<1, 3>(y, o3);
-          lad_gkr<1, 2>(y, [&](int j) { return keep(0, j); }, g[2], g[3], g[4], g[5]);
-          lad_skr<1, 2>(y, o2);
-          input(x, lrole, lpar);
-          lad_g1r<1>(y, [&](int j) { return x[j]; }, g[0], g[1]);
-          lad_s1r<1>(y, c[0], c[1]);
+        if (busy) {
+          get(0);
+          const LadRot p3 = lad_rot<true>(c, 1, 1.0);
+          if (cls == 0) {
+            lad_gkr<0, 3>(y, [&](int j) { return x[j]; }, g[6], g[7], g[8], g[9]);
+            lad_skr<0, 3>(y, p3);
+          } else {
+            lad_gkr<1, 3>(y, [&](int j) { return x[j]; }, g[6], g[7], g[8], g[9]);
+            lad_skr<1, 3>(y, p3);
+          }
+          get(1 + (t & 1));                          // T1 once more: cheaper than a place to keep it
+          const LadRot p2 = lad_rot<true>(c, 0, 1.0);
+          if (cls == 0) {
+            lad_s1r<0>(x, c[0], c[1]);
+            lad_gkr<0, 2>(y, [&](int j) { return x[j]; }, g[2], g[3], g[4], g[5]);
+            lad_skr<0, 2>(y, p2);
+          } else {
+            lad_s1r<1>(x, c[0], c[1]);
+            lad_gkr<1, 2>(y, [&](int j) { return x[j]; }, g[2], g[3], g[4], g[5]);
+            lad_skr<1, 2>(y, p2);
+          }
+          get(1 + (t & 1));
+          if (cls == 0) {
+            lad_g1r<0>(y, [&](int j) { return x[j]; }, g[0], g[1]);
+            lad_s1r<0>(y, c[0], c[1]);
+          } else {
+            lad_g1r<1>(y, [&](int j) { return x[j]; }, g[0], g[1]);
+            lad_s1r<1>(y, c[0], c[1]);
+          }
         }
         __syncwarp();
         swaps = lswaps;
       } else {
-        // w -> (transposed SF, S4) kept, S3 kept, S2: the cotangent at S1's output
-        input(x, rrole, par);
+        // w -> (transposed SF, S4) kept, S3, S2: the cotangent at S1's output
+        get(1 + (t & 1));
         lad_s4r_t(x, r4, lrole, cls, src, u, up, any);
         if (busy) {
-#pragma unroll
-          for (int j = 0; j < NX; ++j) keep(1, j) = x[j];
-        }
-        if (busy && cls == 0) {
-          lad_skr<0, 3>(x, o3);
-#pragma unroll
-          for (int j = 0; j < NX; ++j) keep(0, j) = x[j];
-          lad_skr<0, 2>(x, o2);
-          lad_g1r<0>(x, [&](int j) { return y[j]; }, g[0], g[1]);
-          lad_s1r<0>(y, c[0], c[1]);
-          lad_gkr<0, 2>(y, [&](int j) { return keep(0, j); }, g[2], g[3], g[4], g[5]);
-          lad_skr<0, 2>(y, o2);
-          lad_gkr<0, 3>(y, [&](int j) { return keep(1, j); }, g[6], g[7], g[8], g[9]);
-          lad_skr<0, 3>(y, o3);
-        } else if (busy) {
-          lad_skr<1, 3>(x, o3);
-#pragma unroll
-          for (int j = 0; j < NX; ++j) keep(0, j) = x[j];
-          lad_skr<1, 2>(x, o2);
-          lad_g1r<1>(x, [&](int j) { return y[j]; }, g[0], g[1]);
-          lad_s1r<1>(y, c[0], c[1]);
-          lad_gkr<1, 2>(y, [&](int j) { return keep(0, j); }, g[2], g[3], g[4], g[5]);
-          lad_skr<1, 2>(y, o2);
-          lad_gkr<1, 3>(y, [&](int j) { return keep(1, j); }, g[6], g[7], g[8], g[9]);
-          lad_skr<1, 3>(y, o3);
+          put();
+          const LadRot o3 = lad_rot<true>(c, 1, 1.0), o2 = lad_rot<true>(c, 0, 1.0);
+          if (cls == 0) {
+            lad_skr<0, 3>(x, o3);
+            lad_skr<0, 2>(x, o2);
+            lad_g1r<0>(x, [&](int j) { return y[j]; }, g[0], g[1]);
+            lad_s1r<0>(y, c[0], c[1]);
+          } else {
+            lad_skr<1, 3>(x, o3);
+            lad_skr<1, 2>(x, o2);
+            lad_g1r<1>(x, [&](int j) { return y[j]; }, g[0], g[1]);
+            lad_s1r<1>(y, c[0], c[1]);
+          }
+          get(0);
+          const LadRot q3 = lad_rot<true>(c, 1, 1.0), p2 = lad_rot<true>(c, 0, 1.0);
+          if (cls == 0) {
+            lad_skr<0, 3>(x, q3);
+            lad_gkr<0, 2>(y, [&](int j) { return x[j]; }, g[2], g[3], g[4], g[5]);
+            lad_skr<0, 2>(y, p2);
+          } else {
+            lad_skr<1, 3>(x, q3);
+            lad_gkr<1, 2>(y, [&](int j) { return x[j]; }, g[2], g[3], g[4], g[5]);
+            lad_skr<1, 2>(y, p2);
+          }
+          get(0);
+          const LadRot p3 = lad_rot<true>(c, 1, 1.0);
+          if (cls == 0) {
+            lad_gkr<0, 3>(y, [&](int j) { return x[j]; }, g[6], g[7], g[8], g[9]);
+            lad_skr<0, 3>(y, p3);
+          } else {
+            lad_gkr<1, 3>(y, [&](int j) { return x[j]; }, g[6], g[7], g[8], g[9]);
+            lad_skr<1, 3>(y, p3);
+          }
         }
         __syncwarp();
         // T3 = y; w again; S4 forwards with its products, W, SF
-        input(x, rrole, par);
+        get(1 + (t & 1));
         if (any) {
           lad_for<16>([&](auto G) {
             constexpr int k = decltype(G)::v;
@@ -454,14 +517,15 @@ ladder_back_kernel(LadBackParams p) {
       g[13] = hi ? ga : 0.0;
       g[14] = iz ? 0.0 : gw;
       g[15] = iz ? gw : 0.0;
+      flush(0);
     } else {
       double x[NX];
       const bool iz = q == 0 || q == 3;
       const bool hi = q >= 2;
-      const LadRot o2 = lad_rot<false>(c, 0, 1.0), o3 = lad_rot<false>(c, 1, 1.0), o4 = lad_rot<false>(c, 2, 1.0);
-      const LadS4 r4 = lad_s4_rows<false>(o4, q);
-      const LadRot t2 = lad_rot<false>(c, 0, -1.0), t3 = lad_rot<false>(c, 1, -1.0);
-      const LadSF fwd = lad_sf_row<false>(c, q, code, 1.0), bwd = lad_sf_row<false>(c, q, code, -1.0);
+      const double *in = input_at(rec, on ? w : 0, q);
+      auto rot = [&](int k, double ysign) { return lad_rot<false>(c, k, ysign); };   // read where it is used
+      auto r4 = [&] { return lad_s4_rows<false>(rot(2, 1.0), q); };
+      auto sf = [&](double tsign) { return lad_sf_row<false>(c, q, code, tsign); };
       const double psign = q == 3 ? -1.0 : 1.0;      // lane Z receives -y of lane Y; lane Y +y of lane Z
       // products of S4's output cotangent w4 (own) with its input T3 (own, and the partner's)
       auto g4 = [&](auto w4, auto t3own, auto t3other) {
@@ -480,10 +544,10 @@ ladder_back_kernel(LadBackParams p) {
         }
         // kept row z (lanes Y, Z); received row x (lanes I, X) or +-y
         if (hi) {
-          g[27] = kx; g[28] = ky; g[29] = kz;
-          g[24] = psign * rx; g[25] = psign * ry; g[26] = psign * rz;
+          g[6] = kx; g[7] = ky; g[8] = kz;
+          g[3] = psign * rx; g[4] = psign * ry; g[5] = psign * rz;
         } else {
-          g[21] = rx; g[22] = ry; g[23] = rz;
+          g[0] = rx; g[1] = ry; g[2] = rz;
         }
       };
       // products of the result's cotangent w5 with T4 for this code's row of W
@@ -496,10 +560,10 @@ ladder_back_kernel(LadBackParams p) {
           d = fma(wv, r, d);
         }
         if (code != 0) {
-          if (iz) g[32] = a;
+          if (iz) g[11] = a;
           else {
-            g[30] = a;
-            g[31] = q == 1 ? d : -d;
+            g[9] = a;
+            g[10] = q == 1 ? d : -d;
           }
         }
       };
@@ -513,85 +577,84 @@ ladder_back_kernel(LadBackParams p) {
         // y parked; t -> T1, T2, T3 kept, T4
 #pragma unroll
         for (int j = 0; j < NX; ++j) keep(4, j) = y[j];
-        input(x, q, 0);
+        lad_get<W>(x, in, q);
         put(0);
         lad_s1c(x, c[0], c[1], c[2]);
         put(1);
-        lad_skc<1, 4, 16>(x, o2);
+        lad_skc<1, 4, 16>(x, rot(0, 1.0));
         put(2);
-        lad_skc<4, 16, 1>(x, o3);
+        lad_skc<4, 16, 1>(x, rot(1, 1.0));
         put(3);
-        lad_s4c(x, r4, true);
+        lad_s4c(x, r4(), true);
         gw(at(4), [&](int j) { return x[j]; });
 #pragma unroll
         for (int j = 0; j < NX; ++j) x[j] = keep(4, j);
-        lad_sf(x, bwd);
+        lad_sf(x, sf(-1.0));
         g4([&](int j) { return x[j]; }, at(3), other3);
-        lad_s4c_t(x, r4, true);
-        lad_gkc<4, 16, 1>([&](int j) { return x[j]; }, at(2), g + 12);
-        lad_skc<4, 16, 1>(x, t3);
+        flush(2 * LAD_GROUP);
+        clear();
+        lad_s4c_t(x, r4(), true);
+        lad_gkc<4, 16, 1>([&](int j) { return x[j]; }, at(2), g);
+        flush(LAD_GROUP);
+        clear();
+        lad_skc<4, 16, 1>(x, rot(1, -1.0));
         lad_gkc<1, 4, 16>([&](int j) { return x[j]; }, at(1), g + 3);
-        lad_skc<1, 4, 16>(x, t2);
+        lad_skc<1, 4, 16>(x, rot(0, -1.0));
         lad_g1c([&](int j) { return x[j]; }, at(0), g);
+        flush(0);
         lad_s1c(x, c[0], -c[1], c[2]);
       } else {
         // y parked; w, then S4's, S3's and S2's output cotangents kept
 #pragma unroll
         for (int j = 0; j < NX; ++j) keep(4, j) = y[j];
-        input(x, q, 0);
-        lad_sf(x, bwd);
+        lad_get<W>(x, in, q);
+        lad_sf(x, sf(-1.0));
         put(3);
-        lad_s4c_t(x, r4, true);
+        lad_s4c_t(x, r4(), true);
         put(2);
-        lad_skc<4, 16, 1>(x, t3);
+        lad_skc<4, 16, 1>(x, rot(1, -1.0));
         put(1);
-        lad_skc<1, 4, 16>(x, t2);
+        lad_skc<1, 4, 16>(x, rot(0, -1.0));
         lad_g1c([&](int j) { return x[j]; }, at(4), g);
 #pragma unroll
         for (int j = 0; j < NX; ++j) x[j] = keep(4, j);
         lad_s1c(x, c[0], c[1], c[2]);
         lad_gkc<1, 4, 16>(at(1), [&](int j) { return x[j]; }, g + 3);
-        lad_skc<1, 4, 16>(x, o2);
-        lad_gkc<4, 16, 1>(at(2), [&](int j) { return x[j]; }, g + 12);
-        lad_skc<4, 16, 1>(x, o3);
+        flush(0);
+        clear();
+        lad_skc<1, 4, 16>(x, rot(0, 1.0));
+        lad_gkc<4, 16, 1>(at(2), [&](int j) { return x[j]; }, g);
+        flush(LAD_GROUP);
+        clear();
+        lad_skc<4, 16, 1>(x, rot(1, 1.0));
         g4(at(3), [&](int j) { return x[j]; }, other3);
-        lad_s4c(x, r4, true);
+        lad_s4c(x, r4(), true);
         put(0);
-        input(x, q, 0);
+        lad_get<W>(x, in, q);
         gw([&](int j) { return x[j]; }, at(0));
+        flush(2 * LAD_GROUP);
 #pragma unroll
         for (int j = 0; j < NX; ++j) x[j] = keep(0, j);
-        lad_sf(x, fwd);
+        lad_sf(x, sf(1.0));
       }
 #pragma unroll
       for (int j = 0; j < NX; ++j) y[j] = x[j];
-    }
-    // ---- this step's derivatives, summed over the quad
-    {
-      double sums[NG / 4];
-      lad_quad_sums<NG>(g, q, sums);
-      if (on) {
-        double *dst = p.part + ((size_t)(task.step + i) * NG + (NG / 4) * (2 * (q & 1) + (q >> 1))) * B + b;
-#pragma unroll
-        for (int j = 0; j < NG / 4; ++j) dst[(size_t)j * B] = sums[j];
-      }
     }
     // ---- where the cotangent goes
     fresh = rec.cot_out != -1;
     if (on && rec.cot_out >= 0) {
       role = REAL ? lad_role(q, swaps) : q;
-      const int opar = par;                          // parity where the input lies
-      const bool all = !REAL || !(opar ^ (role == 2));
-      double *dst = cots + ((size_t)(rec.cot_out >> 1) * (4 * NX) + role * NX) * B;
-      if (rec.cot_out & 1) {
+      double *dst = cots + (rec.cot_out >> 1) * slot_size;
+      if (!(rec.cot_out & 1)) {
+        const double2 *src = lad_at<W, NX>(dst, role);
 #pragma unroll
-        for (int j = 0; j < NX; ++j)
-          if (j < 28 || all) dst[(size_t)j * B] = y[j];
-      } else {
-#pragma unroll
-        for (int j = 0; j < NX; ++j)
-          if (j < 28 || all) dst[(size_t)j * B] += y[j];
+        for (int i = 0; i < NX / 2; ++i) {
+          const double2 v = src[lad_stride<W>() * i];
+          y[2 * i] += v.x;
+          y[2 * i + 1] += v.y;
+        }
       }
+      lad_put<W>(y, dst, role);
     }
     __syncwarp();
   }
@@ -609,10 +672,10 @@ ladder_site_sum_kernel(const double *__restrict__ part, const int32_t *__restric
   constexpr int NO = REAL ? 18 : 39;
   __shared__ double red[32][33];
   const int site = blockIdx.x, o = blockIdx.y;
-  int g = o, lo = site_off[4 * site], hi = site_off[4 * site + 4];
+  int g = !REAL && o >= 21 ? o + 3 : o, lo = site_off[4 * site], hi = site_off[4 * site + 4];
   if (o >= STAGE) {
     const int row = (o - STAGE) / NW, code = REAL ? (row == 0 ? 1 : 3) : row + 1;
-    g = STAGE + (o - STAGE) % NW;
+    g = (REAL ? STAGE : STAGE + 3) + (o - STAGE) % NW;
     lo = site_off[4 * site + code];
     hi = site_off[4 * site + code + 1];
   }
