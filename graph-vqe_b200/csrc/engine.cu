@@ -357,7 +357,7 @@ struct vqemps_ctx {
   DevBuf<cplx> grad_sites_t, grad_senv, grad_sbar0, grad_sbar1, grad_rootbar, grad_partial_s, grad_fstate;
   DevBuf<double> grad_stage;
   DevBuf<double> lad_coef, lad_const, lad_poison, lad_envp, lad_envs, lad_theta;
-  DevBuf<double> lad_cotp, lad_cots, lad_part, lad_sums;   // ladder gradients
+  DevBuf<double> lad_cotp, lad_cots, lad_gather, lad_part, lad_sums;   // ladder gradients
   int ladder_list = -1;                 // task list of the ladder kernels, -1: by batch size
   int ladder_launches = 0;              // kernels the last run_ladder launched
   int ladder_B = 0;                     // > 0: the last call ran no gate chain (ladder kernels, bond-doubling

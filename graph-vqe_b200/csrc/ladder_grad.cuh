@@ -27,9 +27,14 @@ struct LadBack {
 
 struct LadClose {
   int32_t slot;      // the word's environment in the other half
-  int32_t flags;     // bit 1: its lanes X and Y count
+  int32_t flags;     // bit 1: its lanes X and Y count, bit 2: a sum made ahead, slot counts those
   double coef;
 };
+struct LadGather {   // a sum of closures made ahead
+  int32_t first, count, slot;
+  int32_t half;      // of the step: 0 takes suffix environments, 1 prefix ones
+};
+constexpr int LAD_CLOSE_MOST = 2, LAD_CLOSE_CHUNK = 16;
 
 constexpr int LAD_GR = 16;   // nx nz | k = 2, 3, 4: xx xz zx zz | W: x z of the step's code
 constexpr int LAD_GC = 36;   // nx ny nz | k = 2: O row-major || k = 3 | 3 unused || k = 4 | W: x y z of the step's code
@@ -43,6 +48,8 @@ struct LadBackParams {
   const LadClose *closers;
   const double *coef;
   const double *envp, *envs;
+  double *gathered;          // sums of closures made ahead, laid out as the environments
+  const LadGather *gathers;
   const double *consts;      // boundaries and zero (LadCoefParams)
   double *cotp, *cots;       // cotangents, laid out as the environments
   double *part;              // [step][LAD_GR or LAD_GC][B]
@@ -154,6 +161,53 @@ __device__ __forceinline__ void lad_quad_sums(const double *g, int q, double *ou
   }
 }
 
+// Sums of many words' closures at one step, which would be one task's serial chain: 12 or 16 lanes per (sum, state), each
+// with a third or a quarter of a digit's pairs, so that four words' loads are in flight. Bound: the latency of
+// loads that depend on the word's record. 64 qubits, 20,000 words, B = 1: the gradient 1,346 -> 530 us with it (the identity
+// chain's steps close 150 words each), 40 qubits, 5,000 words: 437 -> 307 us.
+template <bool REAL, int W>
+__global__ void __launch_bounds__(128)
+ladder_gather_kernel(LadBackParams p, int first, int count) {
+  constexpr int NX = lad_lane_comps<REAL>(), SPLIT = REAL ? 3 : 4, NP = NX / 2 / SPLIT, AHEAD = 4;
+  const long long at = ((long long)blockIdx.x * 128 + threadIdx.x) >> 2, item = at / SPLIT;
+  if (item >= (long long)count * p.B) return;
+  const int q = threadIdx.x & 3, part = (int)(at % SPLIT), b = (int)(item % p.B);
+  const LadGather g = p.gathers[first + item / p.B];
+  const size_t slot_size = (size_t)p.B * (4 * NX), at_b = lad_state<W, NX>(b);
+  const double *other = (g.half ? p.envp : p.envs) + at_b;
+  constexpr int S = lad_stride<W>();
+  double2 x[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) x[i] = make_double2(0.0, 0.0);
+  for (int c = 0; c < g.count; c += AHEAD) {
+    LadClose cl[AHEAD];
+    double2 v[AHEAD][NP];
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) {
+      cl[k] = p.closers[g.first + min(c + k, g.count - 1)];
+      if (c + k >= g.count) cl[k].coef = 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) {
+      const bool use = c + k < g.count && ((cl[k].flags & 2) || q == 0 || q == 3);
+      const double2 *src = lad_at<W, NX>(((cl[k].flags & 4) ? p.gathered + at_b : other) + cl[k].slot * slot_size, q) +
+                           S * NP * part;
+#pragma unroll
+      for (int i = 0; i < NP; ++i) v[k][i] = use ? src[S * i] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k)
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        x[i].x = fma(cl[k].coef, v[k][i].x, x[i].x);
+        x[i].y = fma(cl[k].coef, v[k][i].y, x[i].y);
+      }
+  }
+  double2 *dst = const_cast<double2 *>(lad_at<W, NX>(p.gathered + at_b + g.slot * slot_size, q)) + S * NP * part;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) dst[S * i] = x[i];
+}
+
 constexpr int LAD_BACK = 32;         // threads: one warp, so that shared memory holds as many as it can
 template <bool REAL> __host__ __device__ constexpr int lad_back_arrays() { return REAL ? 3 * LAD_XR : 5 * LAD_XC; }
 template <bool REAL> __host__ __device__ constexpr size_t lad_back_smem() {
@@ -169,8 +223,8 @@ template <bool REAL> __host__ __device__ constexpr size_t lad_back_smem() {
 // to stay in the instruction cache. Complex: the carried tensor and four members in shared memory (82 KB a
 // warp, two an SM), rotations read where they are used: held for the step they spilled 5 KB a thread.
 // Measured (B200), whole gradient call, 16 x 16 transfer products -> this: 64 qubits, 20,000 words, B = 32:
-// 20,850 -> 3,626 us; 40 qubits, 5,000 words, B = 1: 1,488 -> 437 us; complex, 21 qubits, 790 words, B = 7:
-// 876 -> 322 us.
+// 20,850 -> 3,440 us; 40 qubits, 5,000 words, B = 1: 1,488 -> 307 us; complex, 21 qubits, 790 words, B = 7:
+// 876 -> 316 us.
 template <bool REAL, int W>
 __global__ void __launch_bounds__(LAD_BACK, REAL ? 7 : 2)
 ladder_back_kernel(LadBackParams p) {
@@ -282,7 +336,7 @@ ladder_back_kernel(LadBackParams p) {
       for (int c = rec.close; c < close_end; ++c) {
         const LadClose cl = p.closers[c];
         if (!(cl.flags & 2) && !iz) continue;
-        const double2 *src = lad_at<W, NX>(other + cl.slot * slot_size, role);
+        const double2 *src = lad_at<W, NX>(((cl.flags & 4) ? p.gathered + at_b : other) + cl.slot * slot_size, role);
 #pragma unroll
         for (int i = 0; i < NX / 2; ++i) {
           const double2 v = src[lad_stride<W>() * i];

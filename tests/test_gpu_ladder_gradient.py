@@ -121,3 +121,23 @@ def test_gradient_at_angles_that_are_not_finite(vq):
     assert np.isnan(e[1]) and np.isnan(g[1]).all()
     for b in (0, 2):
         assert e[b] == good[0][b] and np.array_equal(g[b], good[1][b])
+
+
+@pytest.mark.parametrize("gates", [("ry",), ("ry", "rz")])
+@pytest.mark.parametrize("count, B", [(2, 1), (3, 1), (16, 3), (17, 1), (300, 8)])
+def test_many_words_that_close_at_one_step(vq, gates, count, B):
+    """Words in one half close at the identity chain's steps: few directly, more in sums of chunks of
+    16 and sums of those. Against the level kernels."""
+    n = 14
+    rng = np.random.default_rng(count)
+    spec = O.hardware_efficient_spec(n, 3, gates, "linear")
+    tails = sorted({"".join(rng.choice(list("XYZ"), 4)) + "".join(rng.choice(list("IXYZ"), 5))
+                    for _ in range(4 * count)})[:count]
+    words = ["I" * 5 + t for t in tails] + [("I" * 5 + t)[::-1] for t in tails] + ["ZZ" + "I" * 12]
+    coeffs = rng.normal(size=len(words))
+    x = rng.uniform(-np.pi, np.pi, (B, spec["count"]))
+    e, g = _grad(vq, spec, words, coeffs, x)
+    e1, g1 = _grad(vq, spec, words, coeffs, x, variant="dmma")
+    tol = 1e-12 * np.abs(coeffs).sum()
+    np.testing.assert_allclose(e, e1, rtol=0, atol=tol)
+    np.testing.assert_allclose(g, g1, rtol=0, atol=tol)
