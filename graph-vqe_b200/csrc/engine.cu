@@ -59,7 +59,7 @@ struct Hamiltonian {
   std::vector<double> coeffs;            // T
   int nzwords = 0;                       // non-identity I/Z words (independent streams)
   bool split_allowed = true;             // loaded with split evaluation allowed
-  std::unique_ptr<LadderPlan> ladder;    // built on the first call of a ladder circuit
+  std::unique_ptr<LadderPlan> ladder;    // ladder circuits: made at load (ensure_ladder_plan)
   // device copies
   DevGroup *d_groups = nullptr;
   DevNode *d_nodes = nullptr;
@@ -734,6 +734,16 @@ extern "C" int vqemps_bond_dims(const vqemps_ctx *ctx, int *dims) {
 #include "multicut_plan.inc"
 #include "split_plan.inc"
 
+static bool use_ladder(const vqemps_ctx *ctx, const Hamiltonian *h);
+static bool use_ladder_grad(const vqemps_ctx *ctx, const Hamiltonian *h);
+struct MadeLadderPlan {
+  std::unique_ptr<LadderPlan> plan;
+  cudaError_t error = cudaSuccess;
+};
+static MadeLadderPlan make_ladder_plan(int device, const LadderCircuit &lc, int n, int T, const std::vector<uint8_t> &codes,
+                                       const std::vector<double> &coeffs);
+static int take_ladder_plan(vqemps_ctx *ctx, Hamiltonian *h, MadeLadderPlan made);
+
 // ---------------------------------------------------------------------------
 // Hamiltonian plan: one prefix trie over the sorted site-order words, each path
 // cut after its term's last non-identity site.
@@ -777,6 +787,12 @@ extern "C" int vqemps_set_hamiltonian(vqemps_ctx *ctx, const char *words, const 
     if (h->offdiag[t]) h->all_diagonal = false;
   }
   h->coeffs.assign(coeffs, coeffs + T);
+  // the ladder's task lists need only the words, too: a thread of their own beside the tries below (96 qubits,
+  // 40,000 words: made by the first call they took it from 3 to 47 ms; the load takes no longer with them)
+  std::future<MadeLadderPlan> ladder;
+  if (T > 0 && (use_ladder(ctx, h.get()) || use_ladder_grad(ctx, h.get())))
+    ladder = std::async(std::launch::async, make_ladder_plan, ctx->device, std::cref(ctx->ladder), n, T, std::cref(code),
+                        std::cref(h->coeffs));
   std::vector<int32_t> sumidx_shared(T), sumidx_word(T), wl, wlast;
   for (int t = 0; t < T; ++t) {
     sumidx_shared[t] = h->offdiag[t] ? -1 : t;
@@ -921,6 +937,10 @@ extern "C" int vqemps_set_hamiltonian(vqemps_ctx *ctx, const char *words, const 
   h->node_off[n] = (int)h->nodes.size();
   build_split_plan(*h, want_split ? suffix.get() : SuffixTrie{}, code, last, ctx->bonds, ctx->split_mode);
   std::vector<int32_t>().swap(h->term_slot);
+  if (ladder.valid()) {
+    const int rc = take_ladder_plan(ctx, h.get(), ladder.get());
+    if (rc) return rc;
+  }
   // upload: every plan array is a 256-byte aligned slice of ONE device
   // allocation, filled by one copy of a packed host image (tens of separate
   // allocations and copies cost more than the plan build itself at 40,000 terms)
