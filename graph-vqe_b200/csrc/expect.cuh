@@ -53,15 +53,28 @@ __device__ __forceinline__ void right_env_body(const cplx *__restrict__ sb, int 
   // site tile rows padded to 33 elements: the first contraction's 16 rows of a
   // half-warp then fall on distinct banks
   constexpr int AS = 2 * CHI + 1;
-  __shared__ cplx A[CHI * AS];
+  static_assert(SITE_ELEMS == 2 * RIGHT_THREADS, "two site elements a thread");
+  __shared__ cplx tile[2][CHI * AS];
   __shared__ cplx R[ENV_ELEMS];
   __shared__ cplx T[2 * ENV_ELEMS];
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, a0 = (tid >> 5) * AS + (tid & 31), a1 = a0 + RIGHT_THREADS / 32 * AS;
   R[tid] = cmake(tid == 0 ? 1.0 : 0.0, 0.0);
   rb[(size_t)n * ENV_ELEMS + tid] = R[tid];
+  // the sweep is one chain of sites: the next one's tensor is loaded while a site is worked on
+  {
+    const cplx *src = sb + (size_t)(n - 1) * SITE_ELEMS + tid;
+    tile[(n - 1) & 1][a0] = src[0];
+    tile[(n - 1) & 1][a1] = src[RIGHT_THREADS];
+  }
+  __syncthreads();
   for (int s = n - 1; s >= 0; --s) {
-    for (int e = tid; e < SITE_ELEMS; e += RIGHT_THREADS) A[(e >> 5) * AS + (e & 31)] = sb[(size_t)s * SITE_ELEMS + e];
-    __syncthreads();
+    const cplx *A = tile[s & 1];
+    cplx next0 = cmake(0, 0), next1 = cmake(0, 0);
+    if (s > 0) {
+      const cplx *src = sb + (size_t)(s - 1) * SITE_ELEMS + tid;
+      next0 = src[0];
+      next1 = src[RIGHT_THREADS];
+    }
     // T_i[c, b'] = sum_c' R[c,c'] A[b',i,c']
     {
       const int c = tid >> 4, bp = tid & 15;
@@ -92,6 +105,8 @@ __device__ __forceinline__ void right_env_body(const cplx *__restrict__ sb, int 
         mb[ENV_ELEMS + tid] = m1;
       }
     }
+    tile[(s + 1) & 1][a0] = next0;
+    tile[(s + 1) & 1][a1] = next1;
     __syncthreads();
   }
   if (leafslot != nullptr && tid == 0) *leafslot = ok ? R[0].x : 0.0;

@@ -214,6 +214,7 @@ __device__ __forceinline__ void level_real_body(const LevelParams &p, int groups
     bulk_copy_g2s(sm.R, p.right_real + ((size_t)b * (p.n + 1) + p.s + 1) * ENV_ELEMS, ENV_ELEMS * sizeof(double),
                   &sm.bar_cta);
   }
+  if constexpr (PARTS) dependents_launch();
   if (!mbar_wait(&sm.bar_cta, 0, RL_WAIT_TRIES)) {
     if (threadIdx.x == 0) p.status[b] = ST_TIMEOUT;
     mbar_wait(&sm.bar_cta, 0, RL_WAIT_TRIES);
@@ -236,6 +237,7 @@ __device__ __forceinline__ void level_real_body(const LevelParams &p, int groups
   DevGroup grp = p.groups[first];
   DevNode nd{};
   if (lane < grp.nchild) nd = p.nodes[grp.child_begin + lane];
+  if constexpr (PARTS) dependency_wait();            // the level before: environments read and overwritten from here on
   stage_parent_real(p, b, grp, E, bar, lane);
   for (int k = 0; k < count; ++k) {
     const int gidx = first + k * stride;
@@ -496,10 +498,10 @@ right_env_real_kernel(const cplx *__restrict__ sites, int n, cplx *__restrict__ 
                       double *__restrict__ panels_t, const int32_t *__restrict__ st_part,
                       const int32_t *__restrict__ part_n, const int32_t *__restrict__ part_idleaf) {
   constexpr int AS = 2 * CHI + 1;
-  __shared__ double A[CHI * AS];
+  __shared__ double tile[2][CHI * AS];
   __shared__ double R[ENV_ELEMS];
   __shared__ double T[2 * ENV_ELEMS];
-  const int b = blockIdx.x, tid = threadIdx.x;
+  const int b = blockIdx.x, tid = threadIdx.x, a0 = (tid >> 5) * AS + (tid & 31), a1 = a0 + RIGHT_THREADS / 32 * AS;
   // partition sets: n is the widest partition (the stride), nb this state's width
   const int nb = st_part ? part_n[st_part[b]] : n;
   if (st_part) identity_leaf = part_idleaf[st_part[b]];
@@ -510,9 +512,20 @@ right_env_real_kernel(const cplx *__restrict__ sites, int n, cplx *__restrict__ 
   R[tid] = tid == 0 ? 1.0 : 0.0;
   rb[(size_t)nb * ENV_ELEMS + tid] = cmake(R[tid], 0.0);
   rr[(size_t)nb * ENV_ELEMS + rl_swz(tid >> 4, tid & 15)] = R[tid];
+  {
+    const cplx *src = sb + (size_t)(nb - 1) * SITE_ELEMS + tid;
+    tile[(nb - 1) & 1][a0] = src[0].x;
+    tile[(nb - 1) & 1][a1] = src[RIGHT_THREADS].x;
+  }
+  __syncthreads();
   for (int s = nb - 1; s >= 0; --s) {
-    for (int e = tid; e < SITE_ELEMS; e += RIGHT_THREADS) A[(e >> 5) * AS + (e & 31)] = sb[(size_t)s * SITE_ELEMS + e].x;
-    __syncthreads();
+    const double *A = tile[s & 1];
+    double next0 = 0.0, next1 = 0.0;                 // the next site's tensor, loaded while this one is worked on
+    if (s > 0) {
+      const cplx *src = sb + (size_t)(s - 1) * SITE_ELEMS + tid;
+      next0 = src[0].x;
+      next1 = src[RIGHT_THREADS].x;
+    }
     if (panels != nullptr) {
       // panel row a, column i * CHI + c: A[a][i][c]; transposed: row c, column i * CHI + a
       double *pn = panels + ((size_t)b * n + s) * RL_PANEL;
@@ -555,6 +568,8 @@ right_env_real_kernel(const cplx *__restrict__ sites, int n, cplx *__restrict__ 
         mb[ENV_ELEMS + tid] = cmake(m1, 0.0);
       }
     }
+    tile[(s + 1) & 1][a0] = next0;
+    tile[(s + 1) & 1][a1] = next1;
     __syncthreads();
   }
   if (identity_leaf >= 0 && leafval != nullptr && tid == 0)
