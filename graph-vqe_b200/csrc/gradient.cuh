@@ -737,6 +737,7 @@ grad_circuit_kernel(const SiteEvent *__restrict__ events, const int32_t *__restr
 __global__ void grad_param_kernel(const double *__restrict__ slot_grad, int nslots,
                                   const int32_t *__restrict__ off, const int32_t *__restrict__ slots,
                                   int P, double *__restrict__ grad, const int32_t *__restrict__ status) {
+  dependency_wait();
   const int b = blockIdx.y;
   const int pi = blockIdx.x * blockDim.x + threadIdx.x;
   if (pi >= P) return;
