@@ -1,7 +1,7 @@
 // Shared device helpers: FP64 complex arithmetic on double2 and engine constants.
 #pragma once
+#include "dependent.cuh"
 #include <cuda_runtime.h>
-#include <utility>
 #include <stdint.h>
 
 namespace vqemps {
@@ -40,28 +40,5 @@ __device__ __forceinline__ double cabs2(cplx a) { return a.x * a.x + a.y * a.y; 
 
 // Status words written by kernels (mirrors vqemps_status).
 enum : int32_t { ST_OK = 0, ST_INSUFFICIENT = 1, ST_NONFINITE = 2, ST_INVALID = 3, ST_TIMEOUT = 5 };
-
-// Dependent launches (programmatic stream serialization): a kernel launched by launch_dependent may start
-// while the one before it in the stream still runs, once all of that one's CTAs have called dependents_launch
-// or ended. What it reads of earlier kernels' results, and what they may still read, it touches after
-// dependency_wait only (a no-op under a plain launch). Every kernel of a chain waits, so a wait covers the whole
-// chain; the first one is launched plainly.
-__device__ __forceinline__ void dependents_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
-template <typename... P, typename... A>
-inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-}
 
 }  // namespace vqemps

@@ -499,7 +499,6 @@ __global__ void __launch_bounds__(REDUCE_THREADS)
 reduce_kernel(const double *__restrict__ leafval, const double *__restrict__ coef, int nleaf,
               const int32_t *__restrict__ term_leaf, int T, const int32_t *__restrict__ status,
               double *__restrict__ energies, double *__restrict__ per_term) {
-  dependents_launch();
   dependency_wait();
   const int b = blockIdx.x;
   reduce_body(leafval + (size_t)b * nleaf, coef, nleaf, term_leaf, T, status[b] == 0, energies + b,

@@ -186,7 +186,6 @@ template <bool REAL>
 __global__ void __launch_bounds__(256)
 ladder_coef_kernel(LadCoefParams p) {
   const int b = blockIdx.x, B = gridDim.x, tid = threadIdx.x;
-  dependents_launch();
   const double *th = p.theta + (size_t)b * p.P;
   if (p.theta_keep != nullptr)
     for (int i = tid; i < p.P; i += 256) p.theta_keep[(size_t)b * p.P + i] = th[i];
@@ -624,7 +623,6 @@ ladder_path_kernel(LadPathParams p) {
   };
   static_assert(LAD_AHEAD == 3, "the words of four steps are kept");
   uint32_t w0 = word(0), w1 = word(1), w2 = word(2), w3 = word(3);
-  dependents_launch();
   dependency_wait();                                         // the rotations, and earlier launches' environments
   stage(0, w0);
   stage(1, w1);
@@ -801,7 +799,6 @@ ladder_close_kernel(const double *__restrict__ envp, const double *__restrict__ 
     pr = pairs[quad / B];
     b = (int)(quad % B);
   }
-  dependents_launch();
   dependency_wait();
   if (live) {
     if ((pr.flags & 2) || q == 0 || q == 3) {

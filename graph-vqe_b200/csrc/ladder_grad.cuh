@@ -169,7 +169,6 @@ template <bool REAL, int W>
 __global__ void __launch_bounds__(128)
 ladder_gather_kernel(LadBackParams p, int first, int count) {
   constexpr int NX = lad_lane_comps<REAL>(), SPLIT = REAL ? 3 : 4, NP = NX / 2 / SPLIT, AHEAD = 4;
-  dependents_launch();
   dependency_wait();
   const long long at = ((long long)blockIdx.x * 128 + threadIdx.x) >> 2, item = at / SPLIT;
   if (item >= (long long)count * p.B) return;
@@ -294,7 +293,6 @@ ladder_back_kernel(LadBackParams p) {
     rec_next = record(task.nsteps - 2);
   }
   int close_end = live ? p.back[task.step + task.nsteps].close : 0;
-  dependents_launch();
   dependency_wait();
   stage(0, w_now, rec_now, lad_role(q, flips(w_now)));
   double y[NX];                        // the carried cotangent (right end of the step for prefix, left end for suffix)
@@ -729,7 +727,6 @@ ladder_site_sum_kernel(const double *__restrict__ part, const int32_t *__restric
   constexpr int NG = REAL ? LAD_GR : LAD_GC, STAGE = REAL ? 14 : 30, NW = REAL ? 2 : 3;
   constexpr int NO = REAL ? 18 : 39;
   __shared__ double red[32][33];
-  dependents_launch();
   dependency_wait();
   const int site = blockIdx.x, o = blockIdx.y;
   int g = !REAL && o >= 21 ? o + 3 : o, lo = site_off[4 * site], hi = site_off[4 * site + 4];
@@ -777,7 +774,6 @@ template <bool REAL>
 __global__ void __launch_bounds__(128)
 ladder_angle_kernel(LadAngleParams p) {
   constexpr int NO = REAL ? 18 : 39;
-  dependents_launch();
   dependency_wait();
   const int item = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
   if (item >= p.n * (p.layers + 1)) return;

@@ -31,10 +31,14 @@
 #include <vector>
 
 #include "../../include/vqemps_mpnn.h"
+#include "dependent.cuh"
 
 namespace {
 
-constexpr int GM_BM = 64, GM_BN = 128, GM_BK = 32, GM_PAD = 8, GM_THREADS = 128;
+using vqemps::dependency_wait;
+using vqemps::launch_dependent;
+
+constexpr int GM_BN = 128, GM_BK = 32, GM_PAD = 8, GM_THREADS = 128;
 
 // ---- operand views (element (m, k) of A, (k, n) of B) ----------------------
 struct ARow {            // A[m * ld + k]
@@ -128,6 +132,7 @@ __device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], const 
 template <int WM, typename LA, typename LB>
 __global__ void __launch_bounds__(GM_THREADS)
 gemm_bf16_kernel(int M, int N, int K, int k_per_split, LA A, LB B, Epilogue ep) {
+  dependency_wait();
   constexpr int BM = 16 * WM, WN = 4 / WM, NT = 16 / WN;     // tile rows, warps along N, n8 tiles per warp
   constexpr int PA = BM * GM_BK / 2 / GM_THREADS, PB = GM_BN * GM_BK / 2 / GM_THREADS;
   static_assert(GM_THREADS == GM_BN, "a thread stages one column of B");
@@ -249,6 +254,7 @@ gemm_bf16_kernel(int M, int N, int K, int k_per_split, LA A, LB B, Epilogue ep) 
 // out[i] = sum over splits s (in order) of partial[s][i]  (+ accumulate flag)
 __global__ void split_reduce_kernel(const float *__restrict__ partial, int splits, size_t count,
                                     float *__restrict__ out) {
+  dependency_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   float s = 0.f;
@@ -260,6 +266,7 @@ __global__ void split_reduce_kernel(const float *__restrict__ partial, int split
 // A[i] = mean over edges e in [off[i], off[i+1]) of M[e]  (edges sorted by destination)
 __global__ void segment_mean_kernel(const float *__restrict__ Mv, const int32_t *__restrict__ off, int N, int W,
                                     float *__restrict__ out) {
+  dependency_wait();
   const int i = blockIdx.x, c = threadIdx.x;
   if (i >= N || c >= W) return;
   const int b = off[i], e = off[i + 1];
@@ -271,6 +278,7 @@ __global__ void segment_mean_kernel(const float *__restrict__ Mv, const int32_t 
 // S[i] = sum over edges with source i (perm sorted by source) of the message cotangents
 __global__ void segment_sum_perm_kernel(BMsg V, const int32_t *__restrict__ perm, const int32_t *__restrict__ off, int N,
                                         int W, float *__restrict__ out) {
+  dependency_wait();
   const int i = blockIdx.x, c = threadIdx.x;
   if (i >= N || c >= W) return;
   float s = 0.f;
@@ -282,12 +290,14 @@ __global__ void segment_sum_perm_kernel(BMsg V, const int32_t *__restrict__ perm
 // y = x masked by m > 0
 __global__ void relu_mask_kernel(const float *__restrict__ x, const float *__restrict__ m, size_t n,
                                  float *__restrict__ y) {
+  dependency_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) y[i] = m[i] > 0.f ? x[i] : 0.f;
 }
 
 // theta = pi tanh(z)
 __global__ void head_kernel(const float *__restrict__ z, size_t n, float *__restrict__ theta) {
+  dependency_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) theta[i] = 3.14159265358979f * tanhf(z[i]);
 }
@@ -295,6 +305,7 @@ __global__ void head_kernel(const float *__restrict__ z, size_t n, float *__rest
 // dz = dtheta * pi (1 - tanh^2 z), from theta = pi tanh z
 __global__ void head_backward_kernel(const float *__restrict__ theta, const float *__restrict__ dtheta, size_t n,
                                      float *__restrict__ dz) {
+  dependency_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float th = theta[i] * (1.0f / 3.14159265358979f);
@@ -307,6 +318,7 @@ constexpr int LOSS_THREADS = 1024;
 __global__ void loss_kernel(const float *__restrict__ theta, const float *__restrict__ target,
                             const float *__restrict__ weight, int N, int out_per_node, float *__restrict__ loss,
                             float *__restrict__ dtheta) {
+  dependency_wait();
   __shared__ float red[LOSS_THREADS];
   __shared__ float wsum_s;
   const int tid = threadIdx.x;
@@ -341,6 +353,7 @@ __global__ void loss_kernel(const float *__restrict__ theta, const float *__rest
 __global__ void adam_kernel(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
                             float *__restrict__ v, size_t n, float lr, float b1, float b2, float eps, float wd,
                             float c1, float c2) {
+  dependency_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i] + wd * w[i];
@@ -400,26 +413,29 @@ static int fail(vqemps_mpnn *net, int code, const std::string &msg) {
 
 constexpr int GM_TILES = 148;    // fewer tiles of 64 rows than SMs: tiles of 16 rows
 
+// Every kernel of a call but its first is a dependent launch: a training step of 32 graphs (42 kernels) 728 -> 685 us.
 template <typename LA, typename LB>
-static cudaError_t launch_gemm(int M, int N, int K, int per, int z, LA A, LB B, Epilogue ep, cudaStream_t st) {
+static cudaError_t launch_gemm(int M, int N, int K, int per, int z, LA A, LB B, Epilogue ep, cudaStream_t st,
+                               bool first = false) {
   const int cols = (N + GM_BN - 1) / GM_BN;
-  if ((long long)((M + 63) / 64) * cols * z < GM_TILES)
-    gemm_bf16_kernel<1, LA, LB><<<dim3((M + 15) / 16, cols, z), GM_THREADS, 0, st>>>(M, N, K, per, A, B, ep);
-  else
-    gemm_bf16_kernel<4, LA, LB><<<dim3((M + 63) / 64, cols, z), GM_THREADS, 0, st>>>(M, N, K, per, A, B, ep);
+  const bool small = (long long)((M + 63) / 64) * cols * z < GM_TILES;
+  const auto kernel = small ? gemm_bf16_kernel<1, LA, LB> : gemm_bf16_kernel<4, LA, LB>;
+  const dim3 grid(small ? (M + 15) / 16 : (M + 63) / 64, cols, z);
+  if (!first) return launch_dependent(kernel, grid, dim3(GM_THREADS), 0, st, M, N, K, per, A, B, ep);
+  kernel<<<grid, GM_THREADS, 0, st>>>(M, N, K, per, A, B, ep);
   return cudaGetLastError();
 }
 
 template <typename LA, typename LB>
-static cudaError_t gemm(int M, int N, int K, LA A, LB B, Epilogue ep, cudaStream_t st) {
+static cudaError_t gemm(int M, int N, int K, LA A, LB B, Epilogue ep, cudaStream_t st, bool first = false) {
   if (M <= 0 || N <= 0) return cudaSuccess;
-  return launch_gemm(M, N, K, std::max(K, 1), 1, A, B, ep, st);
+  return launch_gemm(M, N, K, std::max(K, 1), 1, A, B, ep, st, first);
 }
 
 // Weight gradient out[M x N] = A^T-view [M x K] times B [K x N] and, in row M of out, the bias
 // gradient (B's column sums), with a fixed split of the K (row) range and an ordered reduction of the
 // partials. The split gives about two CTAs per SM (32 graphs: 1,024 nodes in 16 parts instead of 1, 31,000
-// edges in 97 instead of 30). A training step of 32 graphs: 4,180 -> 726 us, most of it the separate
+// edges in 97 instead of 30). A training step of 32 graphs: 4,180 -> 728 us, most of it the separate
 // column sums, which read every row in one chain of loads.
 template <typename LA, typename LB>
 static int gemm_reduce(vqemps_mpnn *net, int M, int N, int K, LA A, LB B, float *out, cudaStream_t st) {
@@ -434,8 +450,8 @@ static int gemm_reduce(vqemps_mpnn *net, int M, int N, int K, LA A, LB B, float 
   ep.out = net->partial.ptr;
   ep.split_stride = count;
   MPNN_TRY(net, launch_gemm(M, N, K, per, z, A, B, ep, st));
-  split_reduce_kernel<<<grid1(count, 128), 128, 0, st>>>(net->partial.ptr, z, count, out);
-  MPNN_TRY(net, cudaGetLastError());
+  MPNN_TRY(net, launch_dependent(split_reduce_kernel, dim3(grid1(count, 128)), dim3(128), 0, st, net->partial.ptr, z, count,
+                                 out));
   return VQEMPS_MPNN_OK;
 }
 
@@ -541,7 +557,7 @@ extern "C" int vqemps_mpnn_forward(vqemps_mpnn *net, const vqemps_graph *gr, flo
   // encoder
   Epilogue ep{};
   ep.kind = EP_RELU; ep.out = net->X[0].ptr; ep.ldo = W; ep.bias = P + net->o_bin;
-  MPNN_TRY(net, gemm(N, W, net->node_in, ARow{gr->node_feat, net->node_in}, BRow{P + net->o_win, W}, ep, st));
+  MPNN_TRY(net, gemm(N, W, net->node_in, ARow{gr->node_feat, net->node_in}, BRow{P + net->o_win, W}, ep, st, true));
   for (int l = 0; l < L; ++l) {
     if (E > 0) {
       Epilogue em{};
@@ -550,8 +566,8 @@ extern "C" int vqemps_mpnn_forward(vqemps_mpnn *net, const vqemps_graph *gr, flo
                          AGatherCat{net->X[l].ptr, W, gr->edge_src, gr->edge_feat, net->edge_in, W},
                          BRow{P + net->o_wm[l], W}, em, st));
     }
-    segment_mean_kernel<<<N, W, 0, st>>>(net->Mv[l].ptr, gr->dst_off, N, W, net->Agg[l].ptr);
-    MPNN_TRY(net, cudaGetLastError());
+    MPNN_TRY(net, launch_dependent(segment_mean_kernel, dim3(N), dim3(W), 0, st, net->Mv[l].ptr, gr->dst_off, N, W,
+                                   net->Agg[l].ptr));
     Epilogue eu{};
     eu.kind = EP_RESID_RELU; eu.out = net->X[l + 1].ptr; eu.ldo = W; eu.bias = P + net->o_bu[l];
     eu.resid = net->X[l].ptr; eu.ldr = W; eu.relu_out = net->R[l].ptr;
@@ -561,8 +577,8 @@ extern "C" int vqemps_mpnn_forward(vqemps_mpnn *net, const vqemps_graph *gr, flo
   Epilogue eo{};
   eo.kind = EP_STORE; eo.out = net->Z.ptr; eo.ldo = net->out; eo.bias = P + net->o_bo;
   MPNN_TRY(net, gemm(N, net->out, W, ARow{net->X[L].ptr, W}, BRow{P + net->o_wo, net->out}, eo, st));
-  head_kernel<<<grid1((size_t)N * net->out), 256, 0, st>>>(net->Z.ptr, (size_t)N * net->out, net->theta.ptr);
-  MPNN_TRY(net, cudaGetLastError());
+  MPNN_TRY(net, launch_dependent(head_kernel, dim3(grid1((size_t)N * net->out)), dim3(256), 0, st, net->Z.ptr,
+                                 (size_t)N * net->out, net->theta.ptr));
   if (angles_dev)
     MPNN_TRY(net, cudaMemcpyAsync(angles_dev, net->theta.ptr, sizeof(float) * N * net->out,
                                   cudaMemcpyDeviceToDevice, st));
@@ -625,16 +641,16 @@ extern "C" int vqemps_mpnn_backward(vqemps_mpnn *net, const vqemps_graph *gr, co
                        ATGatherCat{net->X[l].ptr, W, gr->edge_src, gr->edge_feat, net->edge_in, W}, dV,
                        grad_dev + net->o_wm[l], st);
       if (rc) return rc;
-      segment_sum_perm_kernel<<<N, W, 0, st>>>(dV, gr->src_perm, gr->src_off, N, W, net->S.ptr);
-      MPNN_TRY(net, cudaGetLastError());
+      MPNN_TRY(net, launch_dependent(segment_sum_perm_kernel, dim3(N), dim3(W), 0, st, dV, gr->src_perm, gr->src_off, N, W,
+                                     net->S.ptr));
       Epilogue es{};
       es.kind = EP_GRAD_X; es.out = net->dX.ptr; es.ldo = W; es.accumulate = 1; es.relu_out = net->dU.ptr; es.mask = below;
       MPNN_TRY(net, gemm(N, W, W, ARow{net->S.ptr, W}, BT{P + net->o_wm[l], W}, es, st));
     } else {
       MPNN_TRY(net, cudaMemsetAsync(grad_dev + net->o_wm[l], 0,
                                     sizeof(float) * ((size_t)(W + net->edge_in) * W + W), st));
-      relu_mask_kernel<<<grid1((size_t)N * W), 256, 0, st>>>(net->dX.ptr, below, (size_t)N * W, net->dU.ptr);
-      MPNN_TRY(net, cudaGetLastError());
+      MPNN_TRY(net, launch_dependent(relu_mask_kernel, dim3(grid1((size_t)N * W)), dim3(256), 0, st, net->dX.ptr, below,
+                                     (size_t)N * W, net->dU.ptr));
     }
   }
   // encoder: X0 = relu(F Win + bin)
