@@ -357,11 +357,12 @@ struct vqemps_ctx {
   DevBuf<cplx> grad_sites_t, grad_senv, grad_sbar0, grad_sbar1, grad_rootbar, grad_partial_s, grad_fstate;
   DevBuf<double> grad_stage;
   DevBuf<double> lad_coef, lad_const, lad_poison, lad_envp, lad_envs, lad_theta;
+  DevBuf<int32_t> sites_status;         // of a chain that vqemps_copy_sites runs
   DevBuf<double> lad_cotp, lad_cots, lad_gather, lad_part, lad_sums;   // ladder gradients
   int ladder_list = -1;                 // task list of the ladder kernels, -1: by batch size
   int ladder_launches = 0;              // kernels the last run_ladder launched
   int ladder_B = 0;                     // > 0: the last call ran no gate chain (ladder kernels, bond-doubling
-                                        // states); angles of that many states are in lad_theta
+                                        // states, gradients); angles of that many states are in lad_theta
   int last_B = 0;
   int forced_variant = -1;              // level kernel variant, -1: autotune
   // Autotuner decisions shared by plans of one size class: (batch-size bucket,
@@ -1147,9 +1148,8 @@ static bool use_quad_chain(vqemps_ctx *ctx, int B) {
   return B <= ctx->quad_clusters;
 }
 
-// The gate chain.
-static int launch_chain(vqemps_ctx *ctx, const double *theta_dev, int B, cudaStream_t st) {
-  ctx->ladder_B = 0;
+// The gate chain; the states' statuses go to status.
+static int launch_chain(vqemps_ctx *ctx, const double *theta_dev, int B, int32_t *status, cudaStream_t st) {
   EvolveParams ep{};
   ep.gates = ctx->d_gates;
   ep.ngates = (int)ctx->gates.size();
@@ -1159,7 +1159,7 @@ static int launch_chain(vqemps_ctx *ctx, const double *theta_dev, int B, cudaStr
   ep.theta = theta_dev;
   ep.sites = ctx->sites.ptr;
   ep.bonds = ctx->bonds_ws.ptr;
-  ep.status = ctx->status.ptr;
+  ep.status = status;
   ep.init0 = ctx->init0;
   ep.init1 = ctx->init1;
   ep.max_bond = ctx->max_bond;
@@ -1215,7 +1215,10 @@ static bool exact_states_at(const vqemps_ctx *ctx, bool doubling_ok, int doubled
 }
 
 static int launch_evolve(vqemps_ctx *ctx, const double *theta_dev, int B, cudaStream_t st) {
-  if (!exact_states_at(ctx, ctx->doubling_ok, ctx->doubled_bond)) return launch_chain(ctx, theta_dev, B, st);
+  if (!exact_states_at(ctx, ctx->doubling_ok, ctx->doubled_bond)) {
+    ctx->ladder_B = 0;
+    return launch_chain(ctx, theta_dev, B, ctx->status.ptr, st);
+  }
   CUDA_TRY(ctx, ctx->lad_theta.ensure((size_t)B * std::max(ctx->P, 1)));
   CUDA_TRY(ctx, cudaMemsetAsync(ctx->status.ptr, 0, sizeof(int32_t) * B, st));
   exact_sites_kernel<<<dim3(ctx->n, B), EXACT_THREADS, 0, st>>>(ctx->d_events, ctx->d_ev_off, ctx->d_mats, theta_dev, ctx->P,
@@ -1847,14 +1850,17 @@ extern "C" int vqemps_copy_sites(vqemps_ctx *ctx, int b, double *sites_host, voi
   if (!ctx || !sites_host || b < 0 || b >= ctx->last_B) return VQEMPS_INVALID;
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = as_stream(stream);
-  if (ctx->ladder_B > 0) {              // the last call ran no gate chain: run it now
+  size_t at = b;
+  if (ctx->ladder_B > 0) {              // the last call ran no gate chain: run it for this state, beside the call's statuses
     if (b >= ctx->ladder_B) return VQEMPS_INVALID;
-    const int rc0 = ensure_state_ws(ctx, ctx->ladder_B);
+    const int rc0 = ensure_state_ws(ctx, 1);
     if (rc0) return rc0;
-    const int rc = launch_chain(ctx, ctx->lad_theta.ptr, ctx->ladder_B, st);
+    CUDA_TRY(ctx, ctx->sites_status.ensure(1));
+    const int rc = launch_chain(ctx, ctx->lad_theta.ptr + (size_t)b * ctx->P, 1, ctx->sites_status.ptr, st);
     if (rc) return rc;
+    at = 0;
   }
-  CUDA_TRY(ctx, cudaMemcpyAsync(sites_host, ctx->sites.ptr + (size_t)b * ctx->n * SITE_ELEMS,
+  CUDA_TRY(ctx, cudaMemcpyAsync(sites_host, ctx->sites.ptr + at * ctx->n * SITE_ELEMS,
                                 sizeof(cplx) * ctx->n * SITE_ELEMS, cudaMemcpyDeviceToHost, st));
   CUDA_TRY(ctx, cudaStreamSynchronize(st));
   return VQEMPS_OK;

@@ -251,8 +251,8 @@ int vqemps_set_evolve_mode(vqemps_ctx *ctx, int mode);
  * n * 16 * 2 * 16 complex (re, im) pairs, site s at offset s * 1024 doubles,
  * element (l, p, r) at ((l * 2 + p) * 16 + r), zero padded beyond the bond dims.
  * Used to check the prepared state against the oracle (synchronises). After a
- * call that ran no gate chain (vqemps_set_evolve_mode) the chain runs here, on
- * that call's angles. */
+ * call that ran no gate chain (vqemps_set_evolve_mode; gradients run none) the chain
+ * runs here, for that call's angles of state b; the call's statuses stay as they are. */
 int vqemps_copy_sites(vqemps_ctx *ctx, int b, double *sites_host, void *stream);
 
 /* Partition sets: K independent circuits of uneven width, parameter count and
