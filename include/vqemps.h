@@ -197,7 +197,9 @@ int vqemps_sampled_energy(vqemps_ctx *ctx, int handle, const double *theta_dev, 
  * cutoffs, 2^layers <= max_bond and split evaluation not switched off, their
  * energies are evaluated from it without preparing site tensors (variant 7;
  * equal to the others to rounding, 1e-12 per term). VQEMPS_LADDER_LIST (0, 1
- * or 2), read by vqemps_create, forces one of its task lists (same bits). */
+ * or 2), read by vqemps_create, forces one of the task lists: energies keep their
+ * bits; derivatives, which a list adds up in an order of its own, are equal to rounding.
+ * Left alone, energies take a list by batch size and gradients one by the Pauli sum. */
 int vqemps_set_level_variant(vqemps_ctx *ctx, int variant);
 int vqemps_level_variant(vqemps_ctx *ctx, int handle, int B, int *variant);
 

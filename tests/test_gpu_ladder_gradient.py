@@ -141,3 +141,33 @@ def test_many_words_that_close_at_one_step(vq, gates, count, B):
     tol = 1e-12 * np.abs(coeffs).sum()
     np.testing.assert_allclose(e, e1, rtol=0, atol=tol)
     np.testing.assert_allclose(g, g1, rtol=0, atol=tol)
+
+
+@pytest.mark.parametrize("gates, n, terms", [(("ry",), 40, 5000), (("ry", "rz"), 30, 3000)])
+def test_default_gradients_do_not_depend_on_the_batch(vq, gates, n, terms):
+    """Problems large enough for each task list to be the fastest at some batch size: the same bits for all."""
+    rng = np.random.default_rng(41)
+    spec = O.hardware_efficient_spec(n, 4, gates, "linear")
+    words, coeffs = W.random_hamiltonian(rng, n, terms, 5)
+    x = rng.uniform(-np.pi, np.pi, (32, spec["count"]))
+    e, g = _grad(vq, spec, words, coeffs, x)
+    for B in (1, 3, 8):
+        eb, gb = _grad(vq, spec, words, coeffs, x[:B])
+        assert np.array_equal(eb, e[:B]) and np.array_equal(gb, g[:B]), B
+
+
+def test_captured_gradient_after_a_larger_batch(vq):
+    """What a call of a larger batch has allocated and made serves a smaller one: it can be captured at once."""
+    spec, words, coeffs, x = W.batched_40q(seed=2, batch=32)
+    eng = vq.Engine(0, 16)
+    eng.set_spec(spec)
+    ham = eng.set_hamiltonian(words, coeffs)
+    th = torch.tensor(x, device=eng.device)
+    e, g = eng.energy_grad(ham, th)
+    small, out = th[:2].clone(), []
+    graph = eng.capture(lambda: out.append(eng.energy_grad(ham, small)), warmup=0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out[0][0], e[:2]) and torch.equal(out[0][1], g[:2])
+    del graph
+    eng.close()
