@@ -233,10 +233,9 @@ struct PartSet {
   int nlevels = 0;
   double flops = 0.0;                                        // one evaluation of every partition
   std::vector<int> bonds;                                    // K x (n_max + 1) allocation bounds
-  bool doubling_ok = true;              // every partition has a bond-doubling state
-  int doubled_bond = 1;
-  SiteEvent *d_events = nullptr;        // its events, K x (n_max + 1) offsets
-  int32_t *d_ev_off = nullptr;
+  int nexact = 0;                       // partitions prepared as exact bond-doubling states
+  SiteEvent *d_events = nullptr;        // their events
+  int32_t *d_ev_off = nullptr;          // K x (n_max + 1) offsets, then K flags: exact
   DevGate *d_gates = nullptr;
   cplx *d_mats = nullptr;
   DevGroup *d_groups = nullptr;
@@ -1207,15 +1206,15 @@ static int launch_chain(vqemps_ctx *ctx, const double *theta_dev, int B, int32_t
 }
 
 // The exact bond-doubling state replaces the chain where the chain's SVDs discard nothing: only
-// adjacent CX, zero cutoffs, doubled bonds within max_bond, and no chain asked for by name. The
+// adjacent CX, zero cutoffs, doubled bonds within max_bond, and no chain asked for by name (evolve_pair). The
 // states are equal (in another gauge), and so are the per-state failures: the rank guard cannot
-// fire, and an angle that is not finite fails its state in both.
-static bool exact_states_at(const vqemps_ctx *ctx, bool doubling_ok, int doubled_bond) {
-  return doubling_ok && ctx->evolve_pair < 0 && ctx->abs_cut == 0.0 && ctx->rel_cut == 0.0 && doubled_bond <= ctx->max_bond;
+// fire, and an angle that is not finite fails its state in both. c: the circuit's context.
+static bool has_exact_states(const vqemps_ctx *c) {
+  return c->doubling_ok && c->abs_cut == 0.0 && c->rel_cut == 0.0 && c->doubled_bond <= c->max_bond;
 }
 
 static int launch_evolve(vqemps_ctx *ctx, const double *theta_dev, int B, cudaStream_t st) {
-  if (!exact_states_at(ctx, ctx->doubling_ok, ctx->doubled_bond)) {
+  if (ctx->evolve_pair >= 0 || !has_exact_states(ctx)) {
     ctx->ladder_B = 0;
     return launch_chain(ctx, theta_dev, B, ctx->status.ptr, st);
   }
@@ -1223,7 +1222,7 @@ static int launch_evolve(vqemps_ctx *ctx, const double *theta_dev, int B, cudaSt
   CUDA_TRY(ctx, cudaMemsetAsync(ctx->status.ptr, 0, sizeof(int32_t) * B, st));
   exact_sites_kernel<<<dim3(ctx->n, B), EXACT_THREADS, 0, st>>>(ctx->d_events, ctx->d_ev_off, ctx->d_mats, theta_dev, ctx->P,
                                                                 ctx->n, ctx->init0, ctx->init1, ctx->sites.ptr, nullptr,
-                                                                nullptr, ctx->status.ptr, ctx->lad_theta.ptr);
+                                                                nullptr, nullptr, ctx->status.ptr, ctx->lad_theta.ptr);
   CUDA_TRY(ctx, cudaGetLastError());
   ctx->evolve_launches = 1;
   ctx->ladder_B = B;

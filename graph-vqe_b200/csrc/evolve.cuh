@@ -93,6 +93,8 @@ struct EvolveParams {
   // Mixed partition sets (the per-partition chain kernels): 1 where partition
   // k's circuit is of real gates (real-arithmetic Jacobi), 0 where complex.
   const int32_t *part_real;
+  // Partitions the chain leaves alone (null: none): 1 where the state is prepared another way.
+  const int32_t *part_skip;
   // Multi-CTA chains of one circuit: the pending one-site products of every
   // two-site gate, [B][ngates][8] (U_s then U_{s+1}), formed beforehand by
   // pending_kernel (null: formed by one thread when the gate is applied).
@@ -777,6 +779,7 @@ __device__ __forceinline__ void evolve_body(const EvolveParams &p) {
   const int tid = threadIdx.x;
   const int b = blockIdx.x;
   const int part = p.st_part ? p.st_part[b] : 0;
+  if (p.part_skip && p.part_skip[part]) return;      // all CTAs of the state
   const bool part_real = MODE == CHAIN_PER_PARTITION && p.part_real[part] != 0;
   const int n = p.st_part ? p.part_n[part] : p.n;
   const int gate_begin = p.st_part ? p.part_gate_off[part] : 0;
@@ -899,6 +902,7 @@ __device__ __forceinline__ void evolve_pair_body(const EvolveParams &p) {
   const int rank = (int)cluster.block_rank();
   const int b = blockIdx.x / K;
   const int part = p.st_part ? p.st_part[b] : 0;
+  if (p.part_skip && p.part_skip[part]) return;      // all CTAs of the state
   const bool part_real = MODE == CHAIN_PER_PARTITION && p.part_real[part] != 0;
   const int n = p.st_part ? p.part_n[part] : p.n;
   const double *theta_b = p.theta + (size_t)b * p.P;

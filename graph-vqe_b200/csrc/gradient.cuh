@@ -93,7 +93,7 @@ __device__ __forceinline__ void event_matrix(const SiteEvent &e, const cplx *mat
 // sincos and the event loop (about 5 us). As a state preparation it replaces the gate chain's serial SVDs wherever
 // they would not truncate: 64 partitions of 8-48 qubits 1,603 us there.
 // Partition sets: state b belongs to partition st_part[b], whose events lie at ev_off rows of
-// stride n + 1. status (optional, zeroed before): a matrix that is not finite fails the state when
+// stride n + 1, and only partitions with part_exact set are prepared. status (optional, zeroed before): a matrix that is not finite fails the state when
 // a CX follows it on its site. keep (optional): a copy of the angles.
 // ---------------------------------------------------------------------------
 constexpr int EXACT_THREADS = 256;
@@ -103,12 +103,12 @@ __global__ void __launch_bounds__(EXACT_THREADS)
 exact_sites_kernel(const SiteEvent *__restrict__ events, const int32_t *__restrict__ ev_off,
                    const cplx *__restrict__ mats, const double *__restrict__ theta, int P, int n, cplx init0, cplx init1,
                    cplx *__restrict__ sites, const int32_t *__restrict__ st_part, const int32_t *__restrict__ part_n,
-                   int32_t *__restrict__ status, double *__restrict__ keep) {
+                   const int32_t *__restrict__ part_exact, int32_t *__restrict__ status, double *__restrict__ keep) {
   __shared__ cplx M[EXACT_EVENTS][4];
   __shared__ int32_t kind[EXACT_EVENTS];
   const int q = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int part = st_part ? st_part[b] : 0;
-  if (st_part && q >= part_n[part]) return;
+  if (st_part && (q >= part_n[part] || !part_exact[part])) return;
   const double *theta_b = theta + (size_t)b * P;
   if (keep != nullptr && q == 0)
     for (int i = tid; i < P; i += EXACT_THREADS) keep[(size_t)b * P + i] = theta_b[i];

@@ -198,3 +198,39 @@ def test_real_partition_sets_equal_the_pinned_engine_bitwise(vq, order):
         e1, pt1 = se.energy(sh, x, per_term=True)
         assert e1.item() == e[k].item()
         assert np.array_equal(pt1.cpu().numpy()[0], pt[k, :len(words)].cpu().numpy())
+
+
+@pytest.mark.parametrize("gates", ["real", "mixed"])
+@pytest.mark.parametrize("order", ["msb", "qubit"])
+def test_sets_of_exact_and_truncating_circuits_equal_sets_of_one(vq, gates, order):
+    """A partition's values do not depend on its neighbours: circuits with a bond-doubling state beside circuits that
+    need the gate chain (a routed CX, five layers), against sets of one, bit for bit."""
+    rng = np.random.default_rng(23)
+    parts = []
+    for k, (n, L) in enumerate([(9, 4), (7, 3), (8, 5), (3, 1), (12, 4)]):
+        spec = O.hardware_efficient_spec(n, L, ("ry", "rz") if gates == "mixed" and k in (1, 2) else ("ry",), "linear")
+        if k == 1:
+            spec = dict(spec, ops=spec["ops"] + [("cx", 0, 2)])
+        words, coeffs = random_hamiltonian(rng, n, 60, 3)
+        parts.append((spec, words, np.asarray(coeffs), rng.uniform(-np.pi, np.pi, spec["count"])))
+    eng = vq.Engine(0, 16)
+    shots, seed = 500, 77
+
+    def run(some, first):
+        ps = _load(vq, eng, some, order)
+        theta = ps.pack_theta([p[3] for p in some], device=eng.device)
+        e, pt = eng.partition_energy(ps, theta, per_term=True)
+        es, pts, bits = eng.partition_sampled_energy(ps, theta, shots, seed + first, "philox", per_term=True, return_bits=True)
+        out = [v.cpu().numpy() for v in (e, pt, es, pts)] + [vq.unpack_bits(bits, ps.n_max)]
+        eng.free_partitions(ps)
+        return out
+    e, pt, es, pts, bits = run(parts, 0)
+    for k, (spec, words, coeffs, x) in enumerate(parts):
+        e1, pt1, es1, pts1, bits1 = run(parts[k:k + 1], k)
+        T, n = len(words), spec["n"]
+        assert e1[0] == e[k] and np.array_equal(pt1[0], pt[k, :T])
+        assert es1[0] == es[k] and np.array_equal(pts1[0], pts[k, :T])
+        assert np.array_equal(bits1[0], bits[k][:, :n])
+        ref = O.dense_expectations(O.dense_statevector(spec, x), words).real
+        np.testing.assert_allclose(pt1[0], ref, rtol=0, atol=1e-11)
+    eng.close()
