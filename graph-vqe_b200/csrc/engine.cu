@@ -369,7 +369,8 @@ struct vqemps_ctx {
   std::map<int, int> tuned_by_shape;
   int grad_checkpoint = 8;              // gradient: keep every 8th level's environments
   int grad_mma = 2;                     // gradient levels: 0 SIMT, 1 FP64 DMMA, 2 DMMA with Gauss forward
-  bool grad_default = true;             // no gradient variant asked for: ladder circuits take the ladder kernels
+  bool grad_default = true;             // no gradient variant or checkpoint interval asked for: ladder circuits take the
+                                        // ladder kernels
   int split_mode = -1;                  // split evaluation: -1 when it saves work, 0 never, 1 always
   int evolve_pair = -1;                 // gate chain: 2 four-CTA clusters (real circuits), 1 two-CTA
                                         // clusters, 0 one CTA, -1 by batch size

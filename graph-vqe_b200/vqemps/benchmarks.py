@@ -111,6 +111,7 @@ def bench_partitions(reps: int = 10):
 
 
 def bench_gradient(reps: int = 3, every=(8, 1), plans=("auto", "off")):
+    """The default kernels, then the level kernels at each checkpoint interval (setting one selects them)."""
     spec, words, coeffs, thetas = W.gradient_64q(seed=0)
     for plan in plans:
         eng = vqemps.Engine(0, 16)
@@ -123,8 +124,9 @@ def bench_gradient(reps: int = 3, every=(8, 1), plans=("auto", "off")):
         th = torch.tensor(thetas, dtype=torch.float64, device=dev)
         B = th.shape[0]
         eng.energy(ham, th)                                    # tunes the level kernel outside the timing
-        for k in every:
-            eng.set_grad_checkpoint(k)
+        for k in (None, *every):
+            if k is not None:
+                eng.set_grad_checkpoint(k)
             free0 = torch.cuda.mem_get_info(dev)[0]
             eng.energy_grad(ham, th)
             torch.cuda.synchronize()

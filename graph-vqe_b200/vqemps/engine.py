@@ -286,12 +286,13 @@ class Engine:
         return out_host
 
     def set_grad_checkpoint(self, every: int):
-        """Keep every `every`-th trie level in the gradient's forward sweep (1: all)."""
+        """Keep every `every`-th trie level in the gradient's forward sweep (1: all). Selects the level kernels
+        for ladder circuits too, whose default kernels keep every environment of a pass."""
         check(self.ctx, self.lib.vqemps_set_grad_checkpoint(self.ctx, int(every)), "set_grad_checkpoint")
 
     def set_grad_variant(self, variant: str):
-        """Gradient level kernels: 'dmma3' (FP64 tensor cores, Gauss forward), 'dmma' or 'simt'. The default is
-        the ladder kernels for ladder circuits (include/vqemps.h) and 'dmma3' for the others."""
+        """Gradient level kernels: 'dmma3' (FP64 tensor cores, Gauss forward), 'dmma' or 'simt'. Until this or
+        set_grad_checkpoint is called, ladder circuits (include/vqemps.h) take the ladder kernels and others 'dmma3'."""
         check(self.ctx, self.lib.vqemps_set_grad_variant(self.ctx, {"simt": 0, "dmma": 1, "dmma3": 2}[variant]),
               "set_grad_variant")
 

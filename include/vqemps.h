@@ -136,8 +136,9 @@ int vqemps_energy_grad_batch(vqemps_ctx *ctx, int handle, const double *theta_de
 /* Environment checkpointing of the gradient (no reference counterpart; the
  * reference bounds memory by 128-term chunks, reverse_mps.py:91-96): the forward
  * sweep keeps every `every`-th level, the backward sweep recomputes the rest one
- * segment at a time. Default 8; 1 keeps every level (no recomputation). The ladder
- * kernels keep every environment of a pass instead and bound a pass to 16 GB. */
+ * segment at a time. Default 8; 1 keeps every level (no recomputation). Setting an
+ * interval selects the level kernels for ladder circuits too (vqemps_set_grad_variant):
+ * the ladder kernels keep every environment of a pass and bound a pass to 16 GB. */
 int vqemps_set_grad_checkpoint(vqemps_ctx *ctx, int every);
 /* Gradient level kernels (no reference counterpart): 0 = SIMT FMA kernels,
  * 1 = FP64 DMMA tensor-core kernels, 2 = DMMA with Gauss's three-product complex
@@ -145,7 +146,7 @@ int vqemps_set_grad_checkpoint(vqemps_ctx *ctx, int every);
  * the real-gate DMMA kernels (one real product per complex one; energies and
  * angle gradients equal variant 1's bit for bit). All give the same values to
  * rounding; VQEMPS_GRAD_VARIANT (simt, dmma, dmma3) selects one at creation.
- * Until a variant is selected, gradients of ladder circuits (see
+ * Until a variant or a checkpoint interval is set, gradients of ladder circuits (see
  * vqemps_set_level_variant) of Pauli sums loaded with split evaluation allowed run
  * the ladder kernels (equal to the others to rounding). */
 int vqemps_set_grad_variant(vqemps_ctx *ctx, int variant);

@@ -171,3 +171,35 @@ def test_captured_gradient_after_a_larger_batch(vq):
     assert torch.equal(out[0][0], e[:2]) and torch.equal(out[0][1], g[:2])
     del graph
     eng.close()
+
+
+def test_checkpointing_asked_for_runs_the_kernels_that_checkpoint(vq):
+    """An interval set by the caller is kept to: the level kernels', bit for bit (vqemps_set_grad_checkpoint)."""
+    spec, words, coeffs, x = W.plain_12q(6)
+    x = np.stack([x, -x])
+    out = []
+    for asked in ((), ("checkpoint",), ("variant",), ("variant", "checkpoint")):
+        eng = vq.Engine(0, 16)
+        eng.set_spec(spec)
+        if "variant" in asked:
+            eng.set_grad_variant("dmma3")
+        if "checkpoint" in asked:
+            eng.set_grad_checkpoint(3)
+        e, g = eng.energy_grad(eng.set_hamiltonian(words, coeffs), x)
+        out.append((e.cpu().numpy(), g.cpu().numpy()))
+        eng.close()
+    for e, g in out[2:]:
+        assert np.array_equal(e, out[1][0]) and np.array_equal(g, out[1][1])
+    assert not np.array_equal(out[0][1], out[1][1])
+    np.testing.assert_allclose(out[0][1], out[1][1], rtol=0, atol=1e-11 * np.abs(coeffs).sum())
+
+
+@pytest.mark.parametrize("gates", [("ry",), ("ry", "rz")])
+def test_gradient_of_sums_without_closures(vq, gates):
+    """Identity words and, with real gates, words with an odd number of Y: nothing to walk, derivatives of zero."""
+    spec = O.hardware_efficient_spec(4, 2, gates, "linear")
+    x = np.random.default_rng(2).uniform(-np.pi, np.pi, (3, spec["count"]))
+    words = ["IIII", "IIII"] + (["YIII", "IYZX"] if gates == ("ry",) else [])
+    e, g = _grad(vq, spec, words, np.arange(1.0, 1.0 + len(words)), x)
+    np.testing.assert_allclose(e, np.full(3, 3.0), rtol=0, atol=1e-14)
+    assert np.array_equal(g, np.zeros_like(g))
