@@ -58,7 +58,7 @@ struct Hamiltonian {
   std::vector<uint8_t> codes;            // T x n site-order Pauli codes
   std::vector<double> coeffs;            // T
   int nzwords = 0;                       // non-identity I/Z words (independent streams)
-  bool split_allowed = true;             // loaded with split evaluation allowed
+  bool split_auto = true;                // loaded with the choice of split evaluation left to the engine
   std::unique_ptr<LadderPlan> ladder;    // ladder circuits: made at load (ensure_ladder_plan)
   // device copies
   DevGroup *d_groups = nullptr;
@@ -759,7 +759,7 @@ extern "C" int vqemps_set_hamiltonian(vqemps_ctx *ctx, const char *words, const 
   auto h = std::make_unique<Hamiltonian>();
   h->n = n;
   h->T = T;
-  h->split_allowed = ctx->split_mode != 0;
+  h->split_auto = ctx->split_mode < 0;
   // site-order codes (buildPauliTermData reverses words for the msb map)
   std::vector<uint8_t> code((size_t)T * n);
   std::vector<int> last(T, -1);

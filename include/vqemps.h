@@ -147,7 +147,7 @@ int vqemps_set_grad_checkpoint(vqemps_ctx *ctx, int every);
  * angle gradients equal variant 1's bit for bit). All give the same values to
  * rounding; VQEMPS_GRAD_VARIANT (simt, dmma, dmma3) selects one at creation.
  * Until a variant or a checkpoint interval is set, gradients of ladder circuits (see
- * vqemps_set_level_variant) of Pauli sums loaded with split evaluation allowed run
+ * vqemps_set_level_variant) of Pauli sums loaded with split evaluation left to the engine run
  * the ladder kernels (equal to the others to rounding). */
 int vqemps_set_grad_variant(vqemps_ctx *ctx, int variant);
 
@@ -195,9 +195,10 @@ int vqemps_sampled_energy(vqemps_ctx *ctx, int handle, const double *theta_dev, 
  * followed by one CX on every bond in chain order, all in one direction, at most
  * four layers (the linear and reverse_linear ansatz) -- have an exact matrix
  * product state that needs no SVD. With no variant or gate chain forced, zero
- * cutoffs, 2^layers <= max_bond and split evaluation not switched off, their
- * energies are evaluated from it without preparing site tensors (variant 7;
- * equal to the others to rounding, 1e-12 per term). VQEMPS_LADDER_LIST (0, 1
+ * cutoffs, 2^layers <= max_bond and split evaluation left to the engine (mode -1 of
+ * vqemps_set_split_mode at the load), their energies are evaluated from it without
+ * preparing site tensors (variant 7; equal to the others to rounding, 1e-12 per
+ * term). VQEMPS_LADDER_LIST (0, 1
  * or 2), read by vqemps_create, forces one of the task lists: energies keep their
  * bits; derivatives, which a list adds up in an order of its own, are equal to rounding.
  * Left alone, energies take a list by batch size and gradients one by the Pauli sum. */
@@ -232,7 +233,8 @@ int vqemps_ladder_info(vqemps_ctx *ctx, int handle, int B, double *info);
  * a prefix trie up to a cut site plus a suffix trie from the cut, each word
  * closed by one dot product of its prefix and suffix environments when that
  * needs fewer node-sites. mode -1 (default): when it saves at least 15 % of the
- * node-sites; 0: never; 1: always, at the best cut. Same values to rounding. */
+ * node-sites; 0: never; 1: always, at the best cut. At 0 and 1 ladder circuits are
+ * evaluated that way too. Same values to rounding. */
 int vqemps_set_split_mode(vqemps_ctx *ctx, int mode);
 
 /* Gate chain (no reference counterpart; the reference applies gates one by one,

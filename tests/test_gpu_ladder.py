@@ -177,3 +177,51 @@ def test_angles_that_are_not_finite(vq):
     e, pt = e.cpu().numpy(), pt.cpu().numpy()
     assert np.isnan(e[1]) and np.isnan(pt[1]).all() and e[0] == good[0] and e[2] == good[2]
     eng.close()
+
+
+def test_split_evaluation_asked_for_runs_as_asked(vq):
+    """vqemps_set_split_mode: 'on' is the split plan and 'off' the prefix plan, for energies, gradients and the analytic
+    words of a shot estimate alike; the ladder kernels answer where the choice is left to the engine."""
+    rng = np.random.default_rng(6)
+    spec = O.hardware_efficient_spec(9, 3, ("ry", "rz"), "linear")
+    words, coeffs = W.random_hamiltonian(rng, 9, 60, 3, z_fraction=0.4)
+    x = rng.uniform(-np.pi, np.pi, (2, spec["count"]))
+    out = {}
+    for mode in ("on", "off", "auto"):
+        eng = vq.Engine(0, 16)
+        eng.set_spec(spec)
+        eng.set_split_mode(mode)
+        ham = eng.set_hamiltonian(words, coeffs)
+        assert (eng.level_variant(ham, 2) == "ladder") == (mode == "auto")
+        assert (eng.plan_stats(ham)["cut"] >= 0) or mode != "on"
+        _, g = eng.energy_grad(ham, x)
+        eng.set_grad_variant("dmma3")
+        _, g3 = eng.energy_grad(ham, x)
+        assert torch.equal(g, g3) == (mode != "auto")
+        _, pt = eng.sampled_energy(ham, x, 300, 5, "philox", "shared", per_term=True)
+        out[mode] = pt.cpu().numpy()
+        eng.close()
+    for mode in ("on", "off"):
+        np.testing.assert_allclose(out[mode], out["auto"], rtol=0, atol=1e-11)
+
+
+def test_autotuner_at_40_qubits(vq):
+    """A circuit that is no ladder (CX in both directions): the level kernels are tuned, among them the real ones."""
+    n, count = 40, 0
+    _, words, coeffs, _ = W.batched_40q(0, batch=1)
+    ops = []
+    for layer in range(4):
+        ops += [("ry", q, count + q) for q in range(n)]
+        ops += [("cx", q, q + 1) if layer % 2 else ("cx", q + 1, q) for q in range(n - 1)]
+        count += n
+    spec = dict(n=n, ops=ops, initial=None, count=count)
+    x = np.random.default_rng(9).uniform(-np.pi, np.pi, (16, count))
+    eng = vq.Engine(0, 16)
+    eng.set_spec(spec)
+    ham = eng.set_hamiltonian(words, coeffs)
+    e = eng.energy(ham, x).cpu().numpy()
+    assert eng.level_variant(ham, 16) in set(vq.Engine.LEVEL_VARIANTS) - {"ladder"}
+    for b in (0, 9):
+        ref = float(np.dot(O.expect_words(O.svd_evolve(spec, x[b], 16), words).real, coeffs))
+        assert abs(e[b] - ref) <= 1e-9 * max(1.0, abs(ref))
+    eng.close()
