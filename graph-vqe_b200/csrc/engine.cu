@@ -359,6 +359,7 @@ struct vqemps_ctx {
   DevBuf<int32_t> sites_status;         // of a chain that vqemps_copy_sites runs
   DevBuf<double> lad_cotp, lad_cots, lad_gather, lad_part, lad_sums;   // ladder gradients
   int ladder_list = -1;                 // task list of the ladder kernels, -1: by batch size
+  size_t ladder_bytes = 0;              // > 0: bound of a pass of the ladder kernels (VQEMPS_LADDER_BYTES)
   int ladder_launches = 0;              // kernels the last run_ladder launched
   int ladder_B = 0;                     // > 0: the last call ran no gate chain (ladder kernels, bond-doubling
                                         // states, gradients); angles of that many states are in lad_theta
@@ -468,6 +469,7 @@ extern "C" int vqemps_create(int device, int max_bond, double abs_cut, double re
   }
   if (const char *v = std::getenv("VQEMPS_LADDER_LIST"))
     if (v[0] >= '0' && v[0] < '0' + LAD_LISTS && v[1] == 0) ctx->ladder_list = v[0] - '0';
+  if (const char *v = std::getenv("VQEMPS_LADDER_BYTES")) ctx->ladder_bytes = (size_t)std::strtoull(v, nullptr, 10);
   // VQEMPS_LEVEL_VARIANT pins the trie-level kernel (a name or an index); the
   // autotuner's timings are meaningless under a serialising profiler.
   if (const char *v = std::getenv("VQEMPS_LEVEL_VARIANT")) {

@@ -138,7 +138,8 @@ int vqemps_energy_grad_batch(vqemps_ctx *ctx, int handle, const double *theta_de
  * sweep keeps every `every`-th level, the backward sweep recomputes the rest one
  * segment at a time. Default 8; 1 keeps every level (no recomputation). Setting an
  * interval selects the level kernels for ladder circuits too (vqemps_set_grad_variant):
- * the ladder kernels keep every environment of a pass and bound a pass to 16 GB. */
+ * the ladder kernels keep every environment of a pass and bound a pass to 16 GB (a
+ * Pauli sum that needs more for one state takes the level kernels). */
 int vqemps_set_grad_checkpoint(vqemps_ctx *ctx, int every);
 /* Gradient level kernels (no reference counterpart): 0 = SIMT FMA kernels,
  * 1 = FP64 DMMA tensor-core kernels, 2 = DMMA with Gauss's three-product complex
@@ -201,7 +202,10 @@ int vqemps_sampled_energy(vqemps_ctx *ctx, int handle, const double *theta_dev, 
  * term). VQEMPS_LADDER_LIST (0, 1
  * or 2), read by vqemps_create, forces one of the task lists: energies keep their
  * bits; derivatives, which a list adds up in an order of its own, are equal to rounding.
- * Left alone, energies take a list by batch size and gradients one by the Pauli sum. */
+ * Left alone, energies take a list by batch size and gradients one by the Pauli sum.
+ * VQEMPS_LADDER_BYTES, read there too, bounds the workspace of their passes (8 GB for
+ * energies, 16 GB for gradients, one state at least; the bits do not depend on it
+ * unless it sends a gradient to the level kernels). */
 int vqemps_set_level_variant(vqemps_ctx *ctx, int variant);
 int vqemps_level_variant(vqemps_ctx *ctx, int handle, int B, int *variant);
 

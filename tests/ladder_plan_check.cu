@@ -131,3 +131,7 @@ extern "C" long long check_ladder_plan(int n, int T, const uint8_t *codes, const
   std::snprintf(msg, size, "%s", fault.c_str());
   return -1;
 }
+
+extern "C" int check_ladder_pass(int B, unsigned long long state, unsigned long long budget) {
+  return ladder_pass(B, state, budget);
+}

@@ -225,3 +225,30 @@ def test_autotuner_at_40_qubits(vq):
         ref = float(np.dot(O.expect_words(O.svd_evolve(spec, x[b], 16), words).real, coeffs))
         assert abs(e[b] - ref) <= 1e-9 * max(1.0, abs(ref))
     eng.close()
+
+
+def test_workspace_budget(vq, monkeypatch):
+    """VQEMPS_LADDER_BYTES: passes of fewer states (one at least) give the same bits; where a gradient's state does not
+    fit, the level kernels answer. A state takes some 220 KB for an energy and 730 KB for a gradient here."""
+    spec, words, coeffs, x = W.plain_12q(3)
+    x = x * np.linspace(0.2, 1.0, 19)[:, None]
+    out = []
+    for budget, variant in ((None, None), (str(1500 << 10), None), (str(7 << 20), None), ("1", None), (None, "dmma3")):
+        monkeypatch.delenv("VQEMPS_LADDER_BYTES", raising=False)
+        if budget:
+            monkeypatch.setenv("VQEMPS_LADDER_BYTES", budget)
+        eng = vq.Engine(0, 16)
+        if variant:
+            eng.set_grad_variant(variant)
+        eng.set_spec(spec)
+        ham = eng.set_hamiltonian(words, coeffs)
+        e, pt = eng.energy(ham, x, per_term=True)
+        eg, g = eng.energy_grad(ham, x)
+        out.append([v.cpu().numpy() for v in (e, pt, eg, g)])
+        eng.close()
+    for got in out[1:]:
+        assert np.array_equal(got[0], out[0][0]) and np.array_equal(got[1], out[0][1])
+    for got in out[1:3]:
+        assert np.array_equal(got[2], out[0][2]) and np.array_equal(got[3], out[0][3])
+    assert np.array_equal(out[3][2], out[4][2]) and np.array_equal(out[3][3], out[4][3])
+    assert not np.array_equal(out[0][3], out[4][3])

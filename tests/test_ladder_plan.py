@@ -29,6 +29,7 @@ def check(tmp_path_factory):
         steps = lib.check_ladder_plan(n, T, codes.ctypes.data_as(ctypes.c_void_p), coeffs.ctypes.data_as(ctypes.c_void_p),
                                       mirror, real, layers, msg, 200)
         return steps, msg.value.decode()
+    run.lib = lib
     return run
 
 
@@ -51,3 +52,13 @@ def test_lists_stay_inside_their_arrays(check, mirror, real):
         for layers in (1, 4):
             steps, fault = check(codes, mirror, real, layers)
             assert steps >= 0, (codes.shape, layers, fault)
+
+
+def test_passes_stay_inside_their_budget(check):
+    size = ctypes.c_ulonglong
+    for state in (1, 1000, 3 << 30):
+        for states in (0, 1, 2, 7, 8, 9, 15, 16, 100):
+            for B in (1, 5, 8, 40):
+                n = check.lib.check_ladder_pass(B, size(state), size(states * state + state // 2))
+                assert 1 <= n <= B and (n <= max(states, 1))
+                assert n == B or n == (states & ~7 if states >= 8 else max(states, 1))
