@@ -269,13 +269,20 @@ template <typename T>
 struct DevBuf {
   T *ptr = nullptr;
   size_t cap = 0;
+  // A buffer that grows takes an eighth more than asked for (64 MB at most, and not where that fails): the next Pauli
+  // sum of a solver's run is often a little larger, and each of a call's buffers costs some 100 us to replace.
   cudaError_t ensure(size_t count) {
     if (count <= cap) return cudaSuccess;
+    const size_t more = cap > 0 ? std::min<size_t>(count / 8, ((size_t)64 << 20) / sizeof(T)) : 0;
     if (ptr) cudaFree(ptr);
     ptr = nullptr; cap = 0;
-    cudaError_t e = cudaMalloc(&ptr, std::max<size_t>(count, 1) * sizeof(T));
-    if (e == cudaSuccess) cap = count;
-    return e;
+    for (size_t size : {count + more, count}) {
+      const cudaError_t e = cudaMalloc(&ptr, std::max<size_t>(size, 1) * sizeof(T));
+      if (e == cudaSuccess) cap = size;
+      if (e != cudaErrorMemoryAllocation || size == count) return e;
+      cudaGetLastError();                             // not the next call's
+    }
+    return cudaSuccess;
   }
   void release() { if (ptr) cudaFree(ptr); ptr = nullptr; cap = 0; }
   DevBuf() = default;
@@ -743,7 +750,14 @@ struct MadeLadderPlan {
   std::unique_ptr<LadderPlan> plan;
   cudaError_t error = cudaSuccess;
 };
-static MadeLadderPlan make_ladder_plan(int device, const LadderCircuit &lc, int n, int T, const std::vector<uint8_t> &codes,
+struct LadderRequest {
+  int device;
+  const LadderCircuit *circuit;
+  bool gradients;                       // with the list for gradients
+  int forced_list;                      // VQEMPS_LADDER_LIST or -1
+};
+static LadderRequest ladder_request(const vqemps_ctx *ctx, const Hamiltonian *h);
+static MadeLadderPlan make_ladder_plan(const LadderRequest &want, int n, int T, const std::vector<uint8_t> &codes,
                                        const std::vector<double> &coeffs);
 static int take_ladder_plan(vqemps_ctx *ctx, Hamiltonian *h, MadeLadderPlan made);
 
@@ -794,7 +808,7 @@ extern "C" int vqemps_set_hamiltonian(vqemps_ctx *ctx, const char *words, const 
   // 40,000 words: made by the first call they took it from 3 to 47 ms; the load takes no longer with them)
   std::future<MadeLadderPlan> ladder;
   if (T > 0 && (use_ladder(ctx, h.get()) || use_ladder_grad(ctx, h.get())))
-    ladder = std::async(std::launch::async, make_ladder_plan, ctx->device, std::cref(ctx->ladder), n, T, std::cref(code),
+    ladder = std::async(std::launch::async, make_ladder_plan, ladder_request(ctx, h.get()), n, T, std::cref(code),
                         std::cref(h->coeffs));
   std::vector<int32_t> sumidx_shared(T), sumidx_word(T), wl, wlast;
   for (int t = 0; t < T; ++t) {

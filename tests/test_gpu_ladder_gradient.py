@@ -203,3 +203,24 @@ def test_gradient_of_sums_without_closures(vq, gates):
     e, g = _grad(vq, spec, words, np.arange(1.0, 1.0 + len(words)), x)
     np.testing.assert_allclose(e, np.full(3, 3.0), rtol=0, atol=1e-14)
     assert np.array_equal(g, np.zeros_like(g))
+
+
+def test_first_gradient_on_the_next_pauli_sum_allocates_nothing(vq):
+    """Its task list is made with the sum, and buffers that have grown once hold a little more: the first call can be
+    captured."""
+    rng = np.random.default_rng(8)
+    spec = O.hardware_efficient_spec(30, 4, ("ry",), "linear")
+    eng = vq.Engine(0, 16)
+    eng.set_spec(spec)
+    th = torch.tensor(rng.uniform(-np.pi, np.pi, (8, spec["count"])), device=eng.device)
+    for terms in (1500, 2600):
+        eng.energy_grad(eng.set_hamiltonian(*W.random_hamiltonian(rng, 30, terms, 5)), th)
+    ham = eng.set_hamiltonian(*W.random_hamiltonian(rng, 30, 2680, 5))
+    out = []
+    graph = eng.capture(lambda: out.append(eng.energy_grad(ham, th)), warmup=0)
+    graph.replay()
+    torch.cuda.synchronize()
+    e, g = eng.energy_grad(ham, th)
+    assert torch.equal(out[0][0], e) and torch.equal(out[0][1], g)
+    del graph
+    eng.close()
