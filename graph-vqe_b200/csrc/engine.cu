@@ -328,6 +328,7 @@ struct vqemps_ctx {
   SiteEvent *d_events = nullptr;
   int32_t *d_ev_off = nullptr, *d_ev_dims = nullptr, *d_slot_off = nullptr, *d_slot_list = nullptr;
   LadderCircuit ladder;                 // the circuit as a ladder (ladder_plan.inc)
+  bool scratch = false;                 // of a partition set, whose own arrays go to the device: circuits are compiled only
   LadGate *d_lad_gates = nullptr;
   int32_t *d_lad_off = nullptr;
   // hamiltonians
@@ -664,43 +665,30 @@ extern "C" int vqemps_set_circuit(vqemps_ctx *ctx, int n, const vqemps_op *ops, 
     }
   }
   mark_sigma_side(gates);
-  // upload
-  cudaFree(ctx->d_gates); ctx->d_gates = nullptr;
-  cudaFree(ctx->d_mats); ctx->d_mats = nullptr;
-  CUDA_TRY(ctx, cudaMalloc(&ctx->d_gates, std::max<size_t>(gates.size(), 1) * sizeof(DevGate)));
-  CUDA_TRY(ctx, cudaMalloc(&ctx->d_mats, std::max<size_t>(mats.size(), 1) * sizeof(cplx)));
-  if (!gates.empty())
-    CUDA_TRY(ctx, cudaMemcpy(ctx->d_gates, gates.data(), gates.size() * sizeof(DevGate), cudaMemcpyHostToDevice));
-  CUDA_TRY(ctx, cudaMemcpy(ctx->d_mats, mats.data(), mats.size() * sizeof(cplx), cudaMemcpyHostToDevice));
-  {
-    PairSched ps = build_pair_schedule(gates, n);
-    auto upi = [&](int32_t *&dst, const std::vector<int32_t> &v) -> cudaError_t {
+  ctx->psched = build_pair_schedule(gates, n);
+  const PairSched qs = build_pair_schedule(gates, n, 4);
+  ctx->qsteps = qs.nsteps;
+  ctx->ladder = doubling_ok && named && !ctx->scratch ? compile_ladder(n, gops, real) : LadderCircuit{};
+  ctx->ladder_B = 0;
+  if (!ctx->scratch) {
+    auto up = [&](auto *&dst, const auto &v) -> cudaError_t {
       cudaFree(dst);
       dst = nullptr;
-      cudaError_t e = cudaMalloc(&dst, std::max<size_t>(v.size(), 1) * sizeof(int32_t));
-      if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(dst, v.data(), v.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+      cudaError_t e = cudaMalloc(&dst, std::max<size_t>(v.size(), 1) * sizeof(v[0]));
+      if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice);
       return e;
     };
-    CUDA_TRY(ctx, upi(ctx->d_sched, ps.sched));
-    CUDA_TRY(ctx, upi(ctx->d_gate_q, ps.gate_q));
-    CUDA_TRY(ctx, upi(ctx->d_qlist, ps.qlist));
-    CUDA_TRY(ctx, upi(ctx->d_tail_off, ps.tail_off));
-    ctx->psched = std::move(ps);
-    const PairSched qs = build_pair_schedule(gates, n, 4);
-    CUDA_TRY(ctx, upi(ctx->d_qsched, qs.sched));
-    ctx->qsteps = qs.nsteps;
-  }
-  ctx->ladder = doubling_ok && named ? compile_ladder(n, gops, real) : LadderCircuit{};
-  ctx->ladder_B = 0;
-  if (ctx->ladder.ok) {
-    const LadderCircuit &lc = ctx->ladder;
-    cudaFree(ctx->d_lad_gates); ctx->d_lad_gates = nullptr;
-    cudaFree(ctx->d_lad_off); ctx->d_lad_off = nullptr;
-    CUDA_TRY(ctx, cudaMalloc(&ctx->d_lad_gates, std::max<size_t>(lc.gates.size(), 1) * sizeof(LadGate)));
-    CUDA_TRY(ctx, cudaMalloc(&ctx->d_lad_off, lc.off.size() * sizeof(int32_t)));
-    if (!lc.gates.empty())
-      CUDA_TRY(ctx, cudaMemcpy(ctx->d_lad_gates, lc.gates.data(), lc.gates.size() * sizeof(LadGate), cudaMemcpyHostToDevice));
-    CUDA_TRY(ctx, cudaMemcpy(ctx->d_lad_off, lc.off.data(), lc.off.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    CUDA_TRY(ctx, up(ctx->d_gates, gates));
+    CUDA_TRY(ctx, up(ctx->d_mats, mats));
+    CUDA_TRY(ctx, up(ctx->d_sched, ctx->psched.sched));
+    CUDA_TRY(ctx, up(ctx->d_gate_q, ctx->psched.gate_q));
+    CUDA_TRY(ctx, up(ctx->d_qlist, ctx->psched.qlist));
+    CUDA_TRY(ctx, up(ctx->d_tail_off, ctx->psched.tail_off));
+    CUDA_TRY(ctx, up(ctx->d_qsched, qs.sched));
+    if (ctx->ladder.ok) {
+      CUDA_TRY(ctx, up(ctx->d_lad_gates, ctx->ladder.gates));
+      CUDA_TRY(ctx, up(ctx->d_lad_off, ctx->ladder.off));
+    }
   }
   ctx->gates = std::move(gates);
   ctx->mats = std::move(mats);
@@ -717,7 +705,7 @@ extern "C" int vqemps_set_circuit(vqemps_ctx *ctx, int n, const vqemps_op *ops, 
   ctx->have_circuit = true;
   ctx->real_circuit = real;
   if (ctx->doubling_ok) ctx->doubling_ok = build_site_events(ctx);
-  if (ctx->doubling_ok) {
+  if (ctx->doubling_ok && !ctx->scratch) {
     const int rc = upload_site_events(ctx);
     if (rc) return rc;
   }
