@@ -516,9 +516,8 @@ __device__ __forceinline__ void lad_s4c_t(double (&x)[LAD_XC], const LadS4 &r, b
   }
 }
 
-// ---- SF and its transpose (tsign -1): value <- u value + v value of lane q ^ 3 --------
+// ---- SF and its transpose (tsign -1): value <- u value + v value of lane q ^ 3 (complex amplitudes) --------
 struct LadSF { double u, v; };
-template <bool REAL>
 __device__ __forceinline__ LadSF lad_sf_row(const double *c, int q, int code, double tsign) {
   LadSF r;
   const bool iz = q == 0 || q == 3;
@@ -527,18 +526,9 @@ __device__ __forceinline__ LadSF lad_sf_row(const double *c, int q, int code, do
     r.v = 0.0;
     return r;
   }
-  double a, bb, cc;                       // row of W for this Pauli: x, y, z
-  if constexpr (REAL) {
-    const double *d = c + 17;
-    a = code == 1 ? d[0] : code == 3 ? d[2] : 0.0;
-    cc = code == 1 ? d[1] : code == 3 ? d[3] : 0.0;
-    bb = code == 2 ? d[4] : 0.0;
-  } else {
-    const double *d = c + 30 + 3 * (code - 1);
-    a = d[0]; bb = d[1]; cc = d[2];
-  }
-  r.u = iz ? 0.0 : a;
-  r.v = iz ? cc : (q == 1 ? tsign * bb : -tsign * bb);
+  const double *d = c + 30 + 3 * (code - 1);          // row of W for this Pauli: x, y, z
+  r.u = iz ? 0.0 : d[0];
+  r.v = iz ? d[2] : (q == 1 ? tsign * d[1] : -tsign * d[1]);
   return r;
 }
 template <int N>
@@ -734,7 +724,7 @@ ladder_path_kernel(LadPathParams p) {
       const bool izlane = q == 0 || q == 3;
       if (suffix) {
         if (__any_sync(LAD_FULL, on && code != 0)) {
-          lad_sf(x, lad_sf_row<false>(c, q, code, -1.0));
+          lad_sf(x, lad_sf_row(c, q, code, -1.0));
         } else if (!izlane) {
 #pragma unroll
           for (int j = 0; j < NX; ++j) x[j] = 0.0;
@@ -760,7 +750,7 @@ ladder_path_kernel(LadPathParams p) {
         if (!any && !izlane) r4.ki = r4.kz = r4.kx = r4.ky = 0.0;
         lad_s4c(x, r4, any);
         if (__any_sync(LAD_FULL, on && code != 0)) {
-          lad_sf(x, lad_sf_row<false>(c, q, code, 1.0));
+          lad_sf(x, lad_sf_row(c, q, code, 1.0));
         } else if (!izlane) {
 #pragma unroll
           for (int j = 0; j < NX; ++j) x[j] = 0.0;

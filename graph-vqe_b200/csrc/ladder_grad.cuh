@@ -30,8 +30,8 @@ struct LadClose {
   int32_t flags;     // bit 1: its lanes X and Y count, bit 2: a sum made ahead, slot counts those
   double coef;
 };
-struct LadGather {   // a sum of closures made ahead
-  int32_t first, count, slot;
+struct LadGather {   // a sum of closures made ahead; its slot is its place in the list
+  int32_t first, count;
   int32_t half;      // of the step: 0 takes suffix environments, 1 prefix ones
 };
 constexpr int LAD_CLOSE_MOST = 2, LAD_CLOSE_CHUNK = 16;
@@ -172,7 +172,8 @@ ladder_gather_kernel(LadBackParams p, int first, int count) {
   const long long at = ((long long)blockIdx.x * 128 + threadIdx.x) >> 2, item = at / SPLIT;
   if (item >= (long long)count * p.B) return;
   const int q = threadIdx.x & 3, part = (int)(at % SPLIT), b = (int)(item % p.B);
-  const LadGather g = p.gathers[first + item / p.B];
+  const int slot = first + (int)(item / p.B);
+  const LadGather g = p.gathers[slot];
   const size_t slot_size = (size_t)p.B * (4 * NX), at_b = lad_state<W, NX>(b);
   const double *other = (g.half ? p.envp : p.envs) + at_b;
   constexpr int S = lad_stride<W>();
@@ -203,7 +204,7 @@ ladder_gather_kernel(LadBackParams p, int first, int count) {
         x[i].y = fma(cl[k].coef, v[k][i].y, x[i].y);
       }
   }
-  double2 *dst = const_cast<double2 *>(lad_at<W, NX>(p.gathered + at_b + g.slot * slot_size, q)) + S * NP * part;
+  double2 *dst = const_cast<double2 *>(lad_at<W, NX>(p.gathered + at_b + slot * slot_size, q)) + S * NP * part;
 #pragma unroll
   for (int i = 0; i < NP; ++i) dst[S * i] = x[i];
 }
@@ -580,7 +581,7 @@ ladder_back_kernel(LadBackParams p) {
       const double *in = input_at(rec, on ? w : 0, q);
       auto rot = [&](int k, double ysign) { return lad_rot<false>(c, k, ysign); };   // read where it is used
       auto r4 = [&] { return lad_s4_rows<false>(rot(2, 1.0), q); };
-      auto sf = [&](double tsign) { return lad_sf_row<false>(c, q, code, tsign); };
+      auto sf = [&](double tsign) { return lad_sf_row(c, q, code, tsign); };
       const double psign = q == 3 ? -1.0 : 1.0;      // lane Z receives -y of lane Y; lane Y +y of lane Z
       // products of S4's output cotangent w4 (own) with its input T3 (own, and the partner's)
       auto g4 = [&](auto w4, auto t3own, auto t3other) {
