@@ -801,22 +801,6 @@ ladder_angle_kernel(LadAngleParams p) {
     for (int i = 0; i < 9; ++i) a[i] = at(o + i);
   }
   const double *th = p.theta + (size_t)b * p.P;
-  const double r2 = 0.70710678118654752440;
-  const cplx had[4] = {cmake(r2, 0), cmake(r2, 0), cmake(r2, 0), cmake(-r2, 0)};
-  auto gate = [&](int g, double *o) {
-    const LadGate lg = p.gates[g];
-    DevGate dg{};
-    dg.mat = lg.mat; dg.rot = lg.rot; dg.param = lg.param; dg.angle = lg.angle;
-    cplx m[4];
-    one_site_matrix(dg, p.mats, th, m);
-    bloch(m, o);
-  };
-  auto left = [&](const double *o, double *m) {               // m <- o m
-    double t[9];
-    for (int r = 0; r < 3; ++r)
-      for (int cc = 0; cc < 3; ++cc) t[3 * r + cc] = o[3 * r] * m[cc] + o[3 * r + 1] * m[3 + cc] + o[3 * r + 2] * m[6 + cc];
-    for (int i = 0; i < 9; ++i) m[i] = t[i];
-  };
   auto left_t = [&](const double *o, double *m) {             // m <- o^T m
     double t[9];
     for (int r = 0; r < 3; ++r)
@@ -825,20 +809,20 @@ ladder_angle_kernel(LadAngleParams p) {
   };
   double o[9];
   if (k < 4 && p.hadamard) {
-    bloch(had, o);
+    bloch_hadamard(o);
     left_t(o, a);
   }
   for (int g = g1 - 1; g >= g0; --g) {
     const LadGate lg = p.gates[g];
     if (lg.slot >= 0) {
       double m[9];
-      if (kk == 0) bloch(p.prep, m);
-      else if (p.hadamard) bloch(had, m);
+      if (kk == 0) bloch_exact(p.prep, m);
+      else if (p.hadamard) bloch_hadamard(m);
       else
         for (int i = 0; i < 9; ++i) m[i] = (i % 4 == 0) ? 1.0 : 0.0;
       for (int h = g0; h <= g; ++h) {
-        gate(h, o);
-        left(o, m);
+        bloch_gate(p.gates[h], p.mats, th, o);
+        bloch_left(o, m);
       }
       // axis x v for every column of m: rows r1, r2 of the plane, d r1 = -r2, d r2 = r1 (cyclic after the axis)
       const int r1 = lg.rot == ROT_X ? 1 : lg.rot == ROT_Y ? 2 : 0, r2i = lg.rot == ROT_X ? 2 : lg.rot == ROT_Y ? 0 : 1;
@@ -846,7 +830,7 @@ ladder_angle_kernel(LadAngleParams p) {
       for (int cc = 0; cc < 3; ++cc) d += a[3 * r2i + cc] * m[3 * r1 + cc] - a[3 * r1 + cc] * m[3 * r2i + cc];
       p.stage[(size_t)b * p.nslots + lg.slot] = d * lg.angle + p.poison[b];
     }
-    gate(g, o);
+    bloch_gate(lg, p.mats, th, o);
     left_t(o, a);
   }
 }

@@ -252,3 +252,34 @@ def test_workspace_budget(vq, monkeypatch):
         assert np.array_equal(got[2], out[0][2]) and np.array_equal(got[3], out[0][3])
     assert np.array_equal(out[3][2], out[4][2]) and np.array_equal(out[3][3], out[4][3])
     assert not np.array_equal(out[0][3], out[4][3])
+
+
+@pytest.mark.parametrize("gates", [("ry",), ("ry", "rz"), ("rx", "h", "s")])
+@pytest.mark.parametrize("pattern", ["linear", "reverse_linear"])
+@pytest.mark.parametrize("order", ["msb", "qubit"])
+def test_clifford_circuits_give_whole_numbers(vq, gates, pattern, order):
+    """At angles of zero every gate's Bloch matrix has entries of 0 and +-1, so every value is -1, 0 or 1 without
+    rounding, whichever axis the bonds take (rotations from half angles or a rounded H leave a bias per layer)."""
+    n, L, ops, k = 40, 4, [], 0
+    pairs = [(q, q + 1) for q in range(n - 1)][::1 if pattern == "linear" else -1]
+    for layer in range(L + 1):
+        for q in range(n):
+            for g in gates:
+                if g in ("h", "s"):
+                    ops.append((g, q))
+                else:
+                    ops.append((g, q, k))
+                    k += 1
+        if layer < L:
+            ops += [("cx", a, b) for a, b in pairs]
+    eng = vq.Engine(0, 16)
+    eng.set_circuit(n, ops, site_order=order)
+    words = _words(np.random.default_rng(3), n, 200)
+    ham = eng.set_hamiltonian(words, np.ones(len(words)))
+    assert eng.level_variant(ham, 1) == "ladder"
+    _, pt = eng.energy(ham, np.zeros((2, eng.P)), per_term=True)
+    v = pt.cpu().numpy()
+    assert np.array_equal(v, np.rint(v)) and np.abs(v).max() == 1.0
+    if gates[0] == "ry":                               # the state stays |0 .. 0>
+        assert np.array_equal(v[0], [float(set(w) <= set("IZ")) for w in words])
+    eng.close()
