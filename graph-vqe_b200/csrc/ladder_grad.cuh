@@ -162,8 +162,8 @@ __device__ __forceinline__ void lad_quad_sums(const double *g, int q, double *ou
 
 // Sums of many words' closures at one step, which would be one task's serial chain: 12 or 16 lanes per (sum, state), each
 // with a third or a quarter of a digit's pairs, so that four words' loads are in flight. Bound: the latency of
-// loads that depend on the word's record. 64 qubits, 20,000 words, B = 1: the gradient 1,346 -> 530 us with it (the identity
-// chain's steps close 150 words each), 40 qubits, 5,000 words: 437 -> 307 us.
+// loads that depend on the word's record. With tasks of single nodes, 64 qubits, 20,000 words, B = 1: the gradient 1,346 ->
+// 530 us with it (the identity chain's steps close 150 words each), 40 qubits, 5,000 words: 437 -> 295 us.
 template <bool REAL, int W>
 __global__ void __launch_bounds__(128)
 ladder_gather_kernel(LadBackParams p, int first, int count) {
@@ -224,8 +224,8 @@ template <bool REAL> __host__ __device__ constexpr size_t lad_back_smem() {
 // to stay in the instruction cache. Complex: the carried tensor and four members in shared memory (82 KB a
 // warp, two an SM), rotations read where they are used: held for the step they spilled 5 KB a thread.
 // Measured (B200), whole gradient call, 16 x 16 transfer products -> this: 64 qubits, 20,000 words, B = 32:
-// 20,850 -> 3,440 us; 40 qubits, 5,000 words, B = 1: 1,488 -> 283 us; complex, 21 qubits, 790 words, B = 7:
-// 876 -> 306 us.
+// 20,850 -> 3,450 us; 40 qubits, 5,000 words, B = 1: 1,488 -> 346 us; complex, 21 qubits, 790 words, B = 7:
+// 876 -> 292 us.
 template <bool REAL, int W>
 __global__ void __launch_bounds__(LAD_BACK, REAL ? 7 : 2)
 ladder_back_kernel(LadBackParams p) {
