@@ -382,7 +382,7 @@ level_real_pf_kernel(LevelParams p, int groups_per_warp) {
 
 // A partition set of circuits of real gates: one DMMA product where the complex work-list kernel
 // issues three (64 partitions of 8-48 qubits, the 48 levels: 1,935 -> 805 us, the whole call 2,182 -> 918;
-// 627 with items that fill a resident wave, dependent launches and the sweep that reads ahead; 661-702 on other boxes).
+// 627 with items that fill a resident wave, dependent launches and the sweep that reads ahead; 661-702 on other GPUs).
 __global__ void __launch_bounds__(RL_WARPS * 32, 5)
 level_real_parts_kernel(LevelParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];

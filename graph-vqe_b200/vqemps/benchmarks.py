@@ -167,7 +167,8 @@ def bench_chain(batches=(1, 16, 64, 128, 256), modes=("auto", "quad", "pair", "c
                 sample_only: bool = False):
     """The benchmark circuit's gate chain (40 qubits, 156 two-site gates) for each
     evolve mode and batch size: the prepare phase of an energy call (CUDA events
-    inside the engine). ``sample_only`` runs one-shot sampling calls instead (gate
+    inside the engine). 'auto' runs no chain for this circuit: its phase is the ladder
+    kernels' rotations, or the exact states when sampling. ``sample_only`` runs one-shot sampling calls instead (gate
     chain, right environments, sampler: no trie-level buffers), for profilers."""
     from vqemps import profiling
     spec, words, coeffs, thetas = W.batched_40q(seed=0, batch=max(batches))
