@@ -539,9 +539,10 @@ __device__ __forceinline__ LadSF lad_sf_row(const double *c, int q, int code, do
     r.v = 0.0;
     return r;
   }
-  const double *d = c + 30 + 3 * (code - 1);          // row of W for this Pauli: x, y, z
-  r.u = iz ? 0.0 : d[0];
-  r.v = iz ? d[2] : (q == 1 ? tsign * d[1] : -tsign * d[1]);
+  const double *d = c + 30 + 3 * (code - 1);          // row of W for this Pauli, read whole by every lane
+  const double x = d[0], y = d[1], z = d[2];
+  r.u = iz ? 0.0 : x;
+  r.v = iz ? z : (q == 1 ? tsign * y : -tsign * y);
   return r;
 }
 template <int N>
