@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <numeric>
 #include <string>
@@ -65,7 +66,7 @@ static void walk(const std::vector<LadTask> &tasks, const std::vector<uint32_t> 
 
 static void check_grad(const LadderPlan &pl, int list, int n) {
   LadderGradPlan g;
-  build_ladder_grad_plan(g, pl, LAD_SUBTREE[list]);
+  build_ladder_grad_plan(g, pl.words, pl.leaf_coef, LAD_SUBTREE[list]);
   const int nslot[2] = {g.nslot_p, g.nslot_s};
   std::vector<uint8_t> stored[2] = {std::vector<uint8_t>(nslot[0], 0), std::vector<uint8_t>(nslot[1], 0)};
   walk(g.tasks, g.steps, g.slots, g.launch, nslot, stored, n);
