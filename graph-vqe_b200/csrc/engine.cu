@@ -7,7 +7,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <functional>
 #include <future>
 #include <array>
 #include <map>
@@ -369,6 +368,7 @@ struct vqemps_ctx {
   DevBuf<double> lad_cotp, lad_cots, lad_gather, lad_part, lad_sums;   // ladder gradients
   int ladder_list = -1;                 // task list of the ladder kernels, -1: by batch size
   size_t ladder_bytes = 0;              // > 0: bound of a pass of the ladder kernels (VQEMPS_LADDER_BYTES)
+  bool took_gradients = false;          // a gradient has run the ladder kernels: later sums are loaded with its list
   int ladder_launches = 0;              // kernels the last run_ladder launched
   int ladder_B = 0;                     // > 0: the last call ran no gate chain (ladder kernels, bond-doubling
                                         // states, gradients); angles of that many states are in lad_theta

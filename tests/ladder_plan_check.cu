@@ -4,7 +4,6 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
-#include <functional>
 #include <memory>
 #include <numeric>
 #include <string>
